@@ -699,7 +699,9 @@ size_t SWESim::footprint_estimate() const {
   // Precomputed inner sums: 64 steps (2 x 64 + 1 points for the k-space solver) x N2 columns x (box
   // rows of H0 and r_a, window rows) x nw2.
   const size_t pre_pts = solver == 1 ? 2 * std::min<size_t>(64, nt_) + 1 : std::min<size_t>(64, nt_);
-  b += pre_pts * N2_ * ((size_t)4 * (np_ + 1) + 12) * w2 * c16;
+  // (The fragment kernel's: 8-column tiles of the elements i <= j, two k-steps per matrix, window coefficients.)
+  const size_t tiles = (w2 + (size_t)m.nw + 7) / 8;
+  b += pre_pts * N2_ * std::max(((size_t)4 * (np_ + 1) + 12) * w2 * c16, (size_t)(4 + 3) * tiles * 512);
   return b;
 }
 

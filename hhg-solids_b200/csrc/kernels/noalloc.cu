@@ -17,6 +17,7 @@
 // corrupt each other's current.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
@@ -44,12 +45,28 @@ int propagate_static_scratch(const SolveTables& t, const GroupTables& gt, const 
     snprintf(why, why_len, "no usable current CUDA device (%s)", cudaGetErrorString(e));
     return -1;
   }
-  const size_t need = (size_t)s.vctas * (size_t)t.nt * 3 * sizeof(double2);
+  // A row of partials per virtual CTA.  The fragment kernel runs several CTAs per SM; where their rows
+  // do not fit, the work is split over fewer virtual CTAs, down to one per SM or per 40 k-points of a
+  // column (the largest tile of the element-group kernel), whichever is fewer.
+  LaunchShape shape = s;
+  if (s.kernel == 5) {
+    int sms = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) {
+      snprintf(why, why_len, "cudaDeviceGetAttribute failed: %s", cudaGetErrorString(e));
+      return -1;
+    }
+    const long least = std::min<long>(sms, (long)t.N2 * ((t.row1 - t.row0 + 39) / 40));
+    const long fit = (long)(kStaticScratchBytes / ((size_t)t.nt * 3 * sizeof(double2)));
+    shape.vctas = (int)std::min<long>(s.vctas, std::max(least, fit));
+    shape.ctas = std::min(s.ctas, shape.vctas);
+  }
+  const size_t need = (size_t)shape.vctas * (size_t)t.nt * 3 * sizeof(double2);
   if (need > kStaticScratchBytes) {
     snprintf(why, why_len,
              "this solve needs %zu bytes of scratch for its current partials (%d CTAs x %d steps x 3 axes); "
              "the allocation-free entry point has %zu bytes: use SWESim_run_simulation instead",
-             need, s.vctas, t.nt, kStaticScratchBytes);
+             need, shape.vctas, t.nt, kStaticScratchBytes);
     return -1;
   }
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -83,7 +100,7 @@ int propagate_static_scratch(const SolveTables& t, const GroupTables& gt, const 
     snprintf(why, why_len, "clearing the static scratch failed: %s", cudaGetErrorString(e));
     return -1;
   }
-  launch_propagate(t, gt, s, rho, static_cast<double2*>(scratch), J, stream);
+  launch_propagate(t, gt, shape, rho, static_cast<double2*>(scratch), J, stream);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     snprintf(why, why_len, "propagation launch failed: %s", cudaGetErrorString(e));

@@ -59,8 +59,7 @@ struct LaunchShape {
   int kernel;      // 0: thread per k-point (FP64, nw <= 2, Hermitian); 1: element groups FP64; 2: element groups mixed;
                    // 3: column tiles, thread per k-point (FP64, nw <= 2, Hermitian); 4: tensor-core fragment
                    // kernel (mixed, 11 or 12 orbitals; variant indexes its shape table); 5: FP64 tensor-core
-                   // fragment kernel (plain form, 11 or 12 orbitals); 6: tile kernel (mixed, 11 or 12 orbitals,
-                   // half a warp per k-point)
+                   // fragment kernel (plain form, 3 to 12 orbitals); 6: tile kernel (mixed; 6, 11 or 12 orbitals)
   int k_per_cta;   // k-points per CTA
   int group;       // threads per k-point
   int threads;     // threads per CTA
@@ -98,6 +97,10 @@ bool plan_propagate(const SolveTables& t, int precision, int sm_count, LaunchSha
 bool plan_group(const SolveTables& t, int precision, int sm_count, LaunchShape* out, char* why, int why_len,
                 int tile_hint = 0);
 int launch_group(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
+                 cudaStream_t stream);
+// FP64 tensor-core fragment kernel (plain form, 3..12 orbitals): false if the solve does not suit it.
+bool plan_dfrag(const SolveTables& t, int sm_count, LaunchShape* out);
+int launch_dfrag(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
                  cudaStream_t stream);
 // Column-tile kernel (nw <= 2, Hermitian, FP64): false if the solve does not suit it.
 bool plan_kcol(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem_max, int parts_hint = 0);

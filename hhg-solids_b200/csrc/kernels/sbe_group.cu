@@ -30,6 +30,7 @@
 #include <cstdlib>
 #include <stdexcept>
 
+#include "dmma.cuh"
 #include "sbe_device.h"
 #include "warp_reduce.cuh"
 
@@ -843,7 +844,6 @@ __device__ __forceinline__ GroupData<Real> group_data(const GroupTables& gt) {
 }
 
 #include "sbe_frag.cuh"
-#include "sbe_dfrag.cuh"
 #include "sbe_mtile.cuh"
 
 // One solve: physical CTA b runs virtual CTAs b, b + gridDim.x, ...
@@ -1159,97 +1159,6 @@ const MtileVariant* find_mtile(const SolveTables& t) {
   return nullptr;
 }
 
-// FP64 tensor-core fragment kernel (plain form): precomputed inner sums, compiled 7x7 box, 8 k-points per CTA.
-template <int NW, int NAX, int NJ, bool KM>
-bool plan_dfrag_t(const SolveTables& t, int sm_count, LaunchShape* out, char* why, int why_len) {
-  using FG = dfrag::Geom<NW, NAX, NJ, KM>;
-  auto kern = dfrag::propagate_dfrag_kernel<NW, NAX, NJ, KM>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG::BYTES) != cudaSuccess) {
-    cudaGetLastError();
-    snprintf(why, why_len, "FP64 fragment kernel: %zu bytes of shared memory not available", FG::BYTES);
-    return false;
-  }
-  int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, FG::KPC * 32, FG::BYTES);
-  if (occ < 1) occ = 1;
-  const long slots = (long)occ * sm_count;
-  const int rows = t.row1 - t.row0;
-  const long ntiles = (long)t.N2 * ((rows + FG::KPC - 1) / FG::KPC);
-  out->kernel = 5;
-  out->kmode = KM ? 1 : 0;
-  out->ept = 8;
-  out->k_per_cta = FG::KPC;
-  out->group = 32;
-  out->threads = FG::KPC * 32;
-  out->ntiles = (int)ntiles;
-  out->ctas = (int)(ntiles < slots ? ntiles : slots);
-  out->vctas = out->ctas;
-  out->box_sm = out->win_sm = 0;
-  out->smem = FG::BYTES;
-  out->pre_chunk = std::min(kPreChunk, t.nt);
-  const size_t gbytes = (size_t)FG::NBROWS * FG::NW2 * sizeof(double2), wbytes = (size_t)FG::NWROWS * FG::NW2 * sizeof(double2);
-  out->pre_bytes = KM ? (size_t)(2 * out->pre_chunk + 1) * t.N2 * gbytes + (size_t)t.N2 * wbytes
-                      : (size_t)out->pre_chunk * t.N2 * (gbytes + wbytes);
-  return true;
-}
-
-template <int NW, int NAX, int NJ, bool KM>
-int launch_dfrag_t(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
-                   cudaStream_t stream) {
-  using FG = dfrag::Geom<NW, NAX, NJ, KM>;
-  if (!gt.pre || s.pre_chunk <= 0)
-    throw std::runtime_error("FP64 fragment kernel launch: needs its precomputed-sum scratch (GroupTables::pre)");
-  GroupData<double> d = {gt.Xbox64, gt.P64, gt.T1_64, gt.T2_64, gt.Xwin64, gt.P64, gt.T1_64, gt.T2_64, nullptr, nullptr};
-  const size_t gbuf = (size_t)FG::NBROWS * FG::NW2;
-  double2* Gpre = static_cast<double2*>(gt.pre);
-  const size_t npts_max = KM ? 2 * (size_t)s.pre_chunk + 1 : (size_t)s.pre_chunk;
-  double2* GWpre = Gpre + npts_max * t.N2 * gbuf;
-  d.Gpre = Gpre;
-  d.GWpre = GWpre;
-  auto kern = dfrag::propagate_dfrag_kernel<NW, NAX, NJ, KM>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
-  int launches = 0;
-  for (int c0 = t.step0; c0 < t.step1; c0 += s.pre_chunk) {
-    SolveTables tc = t;
-    tc.step0 = c0;
-    tc.step1 = std::min(c0 + s.pre_chunk, t.step1);
-    const int npts = KM ? 2 * (tc.step1 - c0) + 1 : tc.step1 - c0;
-    launch_group_sums<double>(tc, d, 3, 4, FG::NBROWS, FG::NWROWS, Gpre, GWpre, npts, stream);
-    kern<<<s.ctas, s.threads, s.smem, stream>>>(tc, d, s.vctas, rho, Jpart);
-    launches += 2;
-  }
-  return launches;
-}
-
-struct DfragVariant {
-  int nw, nax, nj;
-  bool km;
-  bool (*plan)(const SolveTables&, int, LaunchShape*, char*, int);
-  int (*launch)(const SolveTables&, const GroupTables&, const LaunchShape&, double2*, double2*, cudaStream_t);
-};
-#define HHG_DFRAG_VARIANT(NW, NAX, NJ, KM) \
-  {NW, NAX, NJ, KM, plan_dfrag_t<NW, NAX, NJ, KM>, launch_dfrag_t<NW, NAX, NJ, KM>}
-// (The k-space solver's 12-orbital two-axis shape needs more shared memory than a CTA has: the
-// element-group kernel runs it.)
-const DfragVariant kDfragVariants[] = {
-    HHG_DFRAG_VARIANT(11, 1, 2, false), HHG_DFRAG_VARIANT(11, 2, 2, false), HHG_DFRAG_VARIANT(12, 1, 2, false),
-    HHG_DFRAG_VARIANT(12, 2, 2, false), HHG_DFRAG_VARIANT(11, 1, 2, true),  HHG_DFRAG_VARIANT(11, 2, 2, true),
-    HHG_DFRAG_VARIANT(12, 1, 2, true),
-};
-#undef HHG_DFRAG_VARIANT
-
-// The FP64 fragment variant for a plain-form solve (Hermitian halved 7x7 box; either solver), or
-// null.  HHG_DFRAG=0 turns it off (measurements).
-const DfragVariant* find_dfrag(const SolveTables& t) {
-  if (const char* env = std::getenv("HHG_DFRAG"))
-    if (env[0] == '0') return nullptr;
-  const GroupGeom gg = group_geom(t);
-  if (!t.hermitian || !gg.half || t.b1n != 7 || t.b2n != 7) return nullptr;
-  for (const DfragVariant& v : kDfragVariants)
-    if (v.nw == t.nw && v.nax == t.nax && v.nj == t.nj && v.km == (t.kmode != 0)) return &v;
-  return nullptr;
-}
-
 struct FragVariant {
   int nw, nax, nj, kpc;
   bool (*plan)(const SolveTables&, int, LaunchShape*, char*, int);
@@ -1370,11 +1279,7 @@ const GroupVariant* find_variant(const SolveTables& t, int precision) {
 
 bool plan_group(const SolveTables& t, int precision, int sm_count, LaunchShape* out, char* why, int why_len,
                 int tile_hint) {
-  if (precision == 0)
-    if (const DfragVariant* f = find_dfrag(t)) {
-      out->variant = (int)(f - kDfragVariants);
-      if (f->plan(t, sm_count, out, why, why_len)) return true;
-    }
+  if (precision == 0 && plan_dfrag(t, sm_count, out)) return true;
   if (precision == 1)  // (the opt-in fragment kernel first: HHG_FRAG=1 asks for it)
     if (const FragVariant* f = find_frag(t, tile_hint)) {
       out->variant = (int)(f - kFragVariants);
@@ -1437,7 +1342,7 @@ int launch_group_batch(const LaunchShape& s, const BatchDesc* descs, const int2*
 int launch_group(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
                  cudaStream_t stream) {
   if (s.kernel == 4) return kFragVariants[s.variant].launch(t, gt, s, rho, Jpart, stream);
-  if (s.kernel == 5) return kDfragVariants[s.variant].launch(t, gt, s, rho, Jpart, stream);
+  if (s.kernel == 5) return launch_dfrag(t, gt, s, rho, Jpart, stream);
   if (s.kernel == 6) return kMtileVariants[s.variant].launch(t, gt, s, rho, Jpart, stream);
   if (s.variant >= 0) return kGroupVariants[s.variant].launch(t, gt, s, rho, Jpart, stream);
   if (s.kmode) return launch_group_generic<true>(t, gt, s, rho, Jpart, stream);

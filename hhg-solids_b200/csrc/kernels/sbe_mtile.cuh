@@ -381,9 +381,9 @@ __global__ void __launch_bounds__(128, 3)
 #pragma unroll
             for (int ks = 0; ks < NKS; ++ks) {
               const double2 b = eb < NW2 ? RS[(4 * ks + c4) * NW2 + eb] : dzero;
-              dfrag::dmma(t1, wa[ks].x, b.x);
-              dfrag::dmma(t2, wa[ks].y, -b.y);
-              dfrag::dmma(t3, wa[ks].x + wa[ks].y, b.x - b.y);
+              dmma(t1, wa[ks].x, b.x);
+              dmma(t2, wa[ks].y, -b.y);
+              dmma(t3, wa[ks].x + wa[ks].y, b.x - b.y);
             }
             if (g < 4) {
 #pragma unroll
