@@ -702,6 +702,8 @@ size_t SWESim::footprint_estimate() const {
   // (The fragment kernel's: 8-column tiles of the elements i <= j, two k-steps per matrix, window coefficients.)
   const size_t tiles = (w2 + (size_t)m.nw + 7) / 8;
   b += pre_pts * N2_ * std::max(((size_t)4 * (np_ + 1) + 12) * w2 * c16, (size_t)(4 + 3) * tiles * 512);
+  // Two orbitals: the column tables of 512 steps, two of up to 22 doubles and two axes' coefficients a step.
+  if (m.nw == 2) b += (std::min<size_t>(512, nt_) + 1) * N2_ * (2 * 22 + 2 * 32) * sizeof(double);
   return b;
 }
 

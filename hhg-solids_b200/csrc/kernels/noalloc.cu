@@ -45,23 +45,25 @@ int propagate_static_scratch(const SolveTables& t, const GroupTables& gt, const 
     snprintf(why, why_len, "no usable current CUDA device (%s)", cudaGetErrorString(e));
     return -1;
   }
-  // A row of partials per virtual CTA.  The fragment kernel runs several CTAs per SM; where their rows
-  // do not fit, the work is split over fewer virtual CTAs, down to one per SM or per 40 k-points of a
-  // column (the largest tile of the element-group kernel), whichever is fewer.
+  // A row of partials per virtual CTA.  The fragment kernel and the pair form of the column tiles split a
+  // solve more finely than the kernels they took over from; where their rows do not fit, the solve runs on
+  // fewer virtual CTAs, down to as many as those kernels used: one per SM or per 40 k-points of a column (the
+  // largest tile of the element-group kernel), or the thread-per-k-point kernels' split.
   LaunchShape shape = s;
-  if (s.kernel == 5) {
+  const size_t row = (size_t)t.nt * 3 * sizeof(double2);
+  if ((s.kernel == 5 || (s.kernel == 3 && s.variant == 2)) && s.vctas * row > kStaticScratchBytes) {
     int sms = 0;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) {
       snprintf(why, why_len, "cudaDeviceGetAttribute failed: %s", cudaGetErrorString(e));
       return -1;
     }
-    const long least = std::min<long>(sms, (long)t.N2 * ((t.row1 - t.row0 + 39) / 40));
-    const long fit = (long)(kStaticScratchBytes / ((size_t)t.nt * 3 * sizeof(double2)));
-    shape.vctas = (int)std::min<long>(s.vctas, std::max(least, fit));
+    const int least = s.kernel == 3 ? thread_per_kpt_rows(t, sms)
+                                    : (int)std::min<long>(sms, (long)t.N2 * ((t.row1 - t.row0 + 39) / 40));
+    shape.vctas = std::min(s.vctas, std::max(least, (int)(kStaticScratchBytes / row)));
     shape.ctas = std::min(s.ctas, shape.vctas);
   }
-  const size_t need = (size_t)shape.vctas * (size_t)t.nt * 3 * sizeof(double2);
+  const size_t need = shape.vctas * row;
   if (need > kStaticScratchBytes) {
     snprintf(why, why_len,
              "this solve needs %zu bytes of scratch for its current partials (%d CTAs x %d steps x 3 axes); "

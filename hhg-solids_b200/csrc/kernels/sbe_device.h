@@ -68,12 +68,12 @@ struct LaunchShape {
   int ntiles;      // work tiles
   int box_sm, win_sm;  // element groups: cell tables staged in shared memory
   int ept;             // element groups: matrix elements per thread
-  int variant;         // element groups: compiled shape (-1: runtime-shaped instance); column tiles: 1 when
-                       // the box rows are Hermitian-halved
+  int variant;         // element groups: compiled shape (-1: runtime-shaped instance); column tiles: 2: pairs of
+                       // rows (sbe_kcol.cu), else sbe_kcol_any.cu, 1 when the box rows are Hermitian-halved
   int kmode;           // instance for the k-space solver (SolveTables::kmode)
   size_t smem;     // dynamic shared memory bytes
-  int pre_chunk;     // element groups: > 0 when the inner Wannier sums of every column are precomputed
-                     // by a separate kernel, this many steps per launch pair
+  int pre_chunk;     // > 0 when the inner Wannier sums (or tables) of every column are precomputed by a
+                     // separate kernel, this many steps per launch pair
   size_t pre_bytes;  // scratch those sums need (GroupTables::pre)
 };
 
@@ -104,8 +104,15 @@ int launch_dfrag(const SolveTables& t, const GroupTables& gt, const LaunchShape&
                  cudaStream_t stream);
 // Column-tile kernel (nw <= 2, Hermitian, FP64): false if the solve does not suit it.
 bool plan_kcol(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem_max, int parts_hint = 0);
-void launch_kcol(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
+int launch_kcol(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
                  cudaStream_t stream);
+// Its general form (sbe_kcol_any.cu): one orbital, and boxes that the two-orbital form does not take.
+bool plan_kcol_any(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem_max, int parts_hint = 0);
+void launch_kcol_any(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
+                     cudaStream_t stream);
+// Current-partial rows of the thread-per-k-point kernels' splits of a two-orbital solve: the fewest virtual CTAs the
+// allocation-free entry runs one on.
+int thread_per_kpt_rows(const SolveTables& t, int sm_count);
 // Persistent work-stealing launch over (solve, virtual CTA) items of solves sharing the kernel shape of
 // `s` (same variant, threads); smem = the largest member's.  Returns the grid size.
 int launch_group_batch(const LaunchShape& s, const BatchDesc* descs, const int2* items, int nitems, int* counter,

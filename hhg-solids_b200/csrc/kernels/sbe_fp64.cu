@@ -287,18 +287,32 @@ __global__ void __launch_bounds__(kKptMaxThreads) propagate_kpt_kernel(SolveTabl
   }
 }
 
-// J[a][ti] = (1/Nk) sum_v Jpart[v][ti][a], summed in virtual-CTA order.
-__global__ void reduce_current_kernel(const double2* Jpart, int ctas, int nt, double inv_nk, double2* J) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 3 * nt) return;
-  const int ti = idx / 3, a = idx % 3;
+// J[a][ti] = (1/Nk) sum_v Jpart[v][ti][a]: a block takes 16 (step, axis) values, thread row p of 16 sums the rows
+// v = p, p + 16, ... in order, and the 16 sums are added in order, so the result does not depend on the launch.
+// (One thread per value walking all rows took 80 us for 400 rows of 1024 steps: a chain of dependent loads.)
+constexpr int kRedVals = 16, kRedParts = 16;
+__global__ void __launch_bounds__(kRedVals * kRedParts) reduce_current_kernel(const double2* Jpart, int ctas, int nt,
+                                                                              double inv_nk, double2* J) {
+  __shared__ double2 part[kRedParts][kRedVals];
+  const int x = threadIdx.x % kRedVals, p = threadIdx.x / kRedVals, idx = blockIdx.x * kRedVals + x;
   double2 acc = make_double2(0.0, 0.0);
-  for (int c = 0; c < ctas; ++c) {
-    const double2 v = Jpart[((size_t)c * nt + ti) * 3 + a];
-    acc.x += v.x;
-    acc.y += v.y;
+  if (idx < 3 * nt) {
+#pragma unroll 4
+    for (int c = p; c < ctas; c += kRedParts) {
+      const double2 v = Jpart[(size_t)c * nt * 3 + idx];
+      acc.x += v.x;
+      acc.y += v.y;
+    }
   }
-  J[(size_t)a * nt + ti] = make_double2(acc.x * inv_nk, acc.y * inv_nk);
+  part[p][x] = acc;
+  __syncthreads();
+  if (p == 0 && idx < 3 * nt) {
+    for (int c = 1; c < kRedParts; ++c) {
+      acc.x += part[c][x].x;
+      acc.y += part[c][x].y;
+    }
+    J[(size_t)(idx % 3) * nt + idx / 3] = make_double2(acc.x * inv_nk, acc.y * inv_nk);
+  }
 }
 
 // rho0(k) = U f U^+ for H(k) = sum_cells e^{-ik.R} H0 (no field): the equilibrium of
@@ -442,6 +456,8 @@ double time_fma(int sms) {
   return flops / (ms * 1e-3) / 1e12;
 }
 
+constexpr size_t kThreadKptSmem = 220 * 1024;
+
 size_t kpt_smem(const SolveTables& t, int threads) {
   const int ncw = t.ncell + t.nwin, qrows = t.kmode ? 2 * kRing + 1 : kRing;
   const size_t n2 = (size_t)(t.ncell * t.nw2 * (1 + t.nax) + t.nj * t.nwin * t.nw2 + ncw * threads + qrows * ncw);
@@ -495,9 +511,15 @@ bool plan_kpt(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem_
 
 }  // namespace
 
+int thread_per_kpt_rows(const SolveTables& t, int sm_count) {
+  LaunchShape s{};
+  if (plan_kcol_any(t, sm_count, &s, kThreadKptSmem) && s.ntiles >= sm_count) return s.vctas;
+  return plan_kpt(t, sm_count, &s, kThreadKptSmem) ? s.vctas : 0;
+}
+
 bool plan_propagate(const SolveTables& t, int precision, int sm_count, LaunchShape* out, char* why, int why_len,
                     int tile_hint) {
-  const size_t kSmemMax = 220 * 1024;
+  *out = LaunchShape{};
   if (t.nw < 1 || t.nw > kMaxOrb) {
     snprintf(why, why_len, "num_orb=%d outside the supported range 1..%d", t.nw, kMaxOrb);
     return false;
@@ -511,14 +533,16 @@ bool plan_propagate(const SolveTables& t, int precision, int sm_count, LaunchSha
   // nw <= 2 runs the FP64 thread-per-k-point kernels in both precisions: with 2x2 matrices the FP32
   // element-group kernel is several times slower, so the mixed form gains nothing there.
   if (!force_group && t.hermitian && t.nw <= 2) {
-    // Column tiles when there are enough columns to fill the GPU, else one k-point per thread in
-    // consecutive-k tiles.
+    // Column tiles: the pair form on all but the smallest grids (the thread-per-k-point kernel keeps those of a few
+    // warps, which a test pins, at 1024 steps of 12 x 12 in 1.69 ms against 0.28), the general form when there are
+    // enough columns to fill the GPU; else one k-point per thread in consecutive-k tiles.
     LaunchShape kc{};
-    if (!force_kpt && plan_kcol(t, sm_count, &kc, kSmemMax, tile_hint) && (force_kcol || kc.ntiles >= sm_count)) {
+    if (!force_kpt && plan_kcol(t, sm_count, &kc, kThreadKptSmem, tile_hint) &&
+        (force_kcol || (kc.variant == 2 ? (t.row1 - t.row0) * t.N2 >= 160 : kc.ntiles >= sm_count))) {
       *out = kc;
       return true;
     }
-    if (plan_kpt(t, sm_count, out, kSmemMax)) return true;
+    if (plan_kpt(t, sm_count, out, kThreadKptSmem)) return true;
   }
   return plan_group(t, precision, sm_count, out, why, why_len, tile_hint);
 }
@@ -532,10 +556,7 @@ int launch_propagate_steps(const SolveTables& t, const GroupTables& gt, const La
     kern<<<s.ctas, s.threads, s.smem, stream>>>(t, s.vctas, rho, Jpart);
     return 1;
   }
-  if (s.kernel == 3) {
-    launch_kcol(t, gt, s, rho, Jpart, stream);
-    return 1;
-  }
+  if (s.kernel == 3) return launch_kcol(t, gt, s, rho, Jpart, stream);
   return launch_group(t, gt, s, rho, Jpart, stream);
 }
 
@@ -553,14 +574,14 @@ int launch_propagate(const SolveTables& t, const GroupTables& gt, const LaunchSh
                      double2* J, cudaStream_t stream, cudaEvent_t after_propagate) {
   const int launches = launch_propagate_steps(t, gt, s, rho, Jpart, stream);
   if (after_propagate) record_event(after_propagate, stream);
-  const int n = 3 * t.nt;
-  reduce_current_kernel<<<(n + 255) / 256, 256, 0, stream>>>(Jpart, s.vctas, t.nt, 1.0 / (double)t.Nk, J);
+  launch_reduce_current(Jpart, s.vctas, t.nt, t.Nk, J, stream);
   return launches + 1;
 }
 
 void launch_reduce_current(const double2* Jpart, int vctas, int nt, int Nk, double2* J, cudaStream_t stream) {
   const int n = 3 * nt;
-  reduce_current_kernel<<<(n + 255) / 256, 256, 0, stream>>>(Jpart, vctas, nt, 1.0 / (double)Nk, J);
+  reduce_current_kernel<<<(n + kRedVals - 1) / kRedVals, kRedVals * kRedParts, 0, stream>>>(Jpart, vctas, nt,
+                                                                                            1.0 / (double)Nk, J);
 }
 
 int launch_rho0_fp64(const SolveTables& t, double2* rho, cudaStream_t stream) {

@@ -1,27 +1,50 @@
-// Column-tile FP64 propagation for nw <= 2 with a Hermitian placement (the 2-orbital configurations).
+// Column-tile FP64 propagation for two orbitals with a Hermitian placement and a cell box symmetric about
+// zero and at most 7 x 7 cells (the 2-orbital configurations).
 //
-// Same propagation as propagate_kpt_kernel (the k-space-resident RK4 of src/solver.cpp:86-181 with
-// the current of src/observable.cpp:16-30, or the k-space solver of src/solver_kspace.cpp), with the
-// Wannier sums in separable form shared by a k-grid column:
+// Same propagation as sbe_kcol_any.cu (the k-space-resident RK4 of src/solver.cpp:86-181 with the current of
+// src/observable.cpp:16-30; KM: the k-space solver of src/solver_kspace.cpp).
 //
-//   H(k) = sum_n1 e^{-2 pi i m1 n1 / N1} G(n1),   G(n1) = P1(n1) sum_n2 e^{-2 pi i m2 n2 / N2} P2(n2) X(n1, n2)
+// H = (D, o), D = H00 - H11, o = H01, is all the commutator needs:
+//   k00 = 2 (o.y x.x - o.x x.y) = -k11,  k01 = -i (D x - d o),  x = X01, d = X00 - X11.
+// With t = e^{-2 pi i m1 / N1} and G(-n1) = G(n1)^+ every part of H is T0 + sum_{n1 > 0} (Re t^n1 A(n1) + Im t^n1
+// B(n1)), A and B the same for a whole k-grid column.  Rows m1 and m1 + N1/2 have t^n1 equal for even n1 and
+// opposite for odd, so a thread takes both: the even and the odd half of the sum are formed once.  The same
+// holds for the window's row twiddles in the current: it needs the sum of the pair's states for n1 = 0, +-2 and
+// their difference for n1 = +-1.
 //
-// (P = the per-point factors: Peierls powers e^{i n A.a}, or the k-space solver's interpolation
-// factors) and likewise for the current window.  A CTA owns R consecutive rows m1 of one column m2,
-// one thread per k-point with its state in registers.  Every kRing steps the CTA computes the
-// column's G for all points of the chunk into shared memory (one pair of barriers per chunk); per
-// step each thread then sums the box rows (n1 >= 0 only when the placement is Hermitian and the box
-// symmetric) and 4 window rows with its own row twiddles, instead of every cell of the support and
-// window.
-#include <cstdio>
+// Column tables (column_tables): per k-grid column and step, with the field applied: real-space solver, H at t
+// and t + dt (at t + dt/2 the field is their mean, so the middle stages run on the sum of the two with the factor
+// in the stage's constants); k-space solver, H at t + dt/2 and t + dt; and the window coefficients.
+//
+// A CTA takes a tile of up to 32 pairs of one column for all steps of the launch (propagate_tile), a thread per
+// pair, states in registers.  Every kIv steps it has staged kIv steps of states in shared memory; during the next
+// kIv they are summed over the rows (five real sums per state value; lane = quarter of the rows, step, value pair;
+// the twiddles in registers) and the sums contracted with the window coefficients.  Where the tiles are many one
+// warp does both, without a barrier; where they are few a second warp takes the sums (SPLIT), and the two meet
+// every kIv steps.  The other CTAs of a launch form the next launch's tables, so only a pulse's first ones are
+// waited for.
+//
+// What bounds it: FP64 operations on three different operands take about 3.2 cycles of a sub-partition (register
+// reads; 2.2 with shared operands), 172 of them per pair and step: 550 cycles a step for each tile of the
+// sub-partition with the most tiles.  A lone tile is bound by the chain of its stages (8 cycles to each FP64
+// result).
+//
+// Measured on B200 (1965 MHz), 4096 steps, one field axis: 200 x 200 2.60 ms (one k-point per thread, window and
+// Peierls factors summed per CTA: 4.36), k-space solver 2.49 ms (5.75); 60 x 60 1.05 ms (thread-per-k-point kernel
+// with per-thread cell sums: 6.16).
 #include <algorithm>
+#include <cstdio>
 #include <cstdlib>
+#include <stdexcept>
 
 #include "sbe_device.h"
-#include "sbe_herm2.cuh"
 
 namespace hhg {
 namespace {
+
+constexpr int kIv = 4;          // steps per staged interval
+constexpr int kKcolChunk = 256; // steps per launch
+constexpr int kTabPts = 32;     // evaluation points of a table CTA
 
 __device__ __forceinline__ double2 kc_mul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
@@ -33,477 +56,602 @@ __device__ __forceinline__ double2 kc_fma(double2 a, double2 b, double2 c) {
   c.y = fma(a.y, b.x, c.y);
   return c;
 }
-__device__ __forceinline__ double kc_warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-// Steps per flush of the window-contracted current partials (see the kernel).
-constexpr int kRJ = 16;
-// Row stride (doubles) of a warp's staged state in the current contraction: 32 lanes + 4, so the
-// eight 16-byte pairs one load instruction touches (4 state values x 2 lane halves, the halves
-// interleaved by pairs) fall in distinct banks.
-constexpr int kYS = 36;
-
 __device__ __forceinline__ int kc_wrap(long long x, int n) {
-  int r = (int)(x % n);
+  const int r = (int)(x % n);
   return r < 0 ? r + n : r;
 }
-
-constexpr int kKcolMaxThreads = 256;
-
-// Hermitian halving of the box rows: with H(-n) = H(n)^+ on the grid and a box symmetric about
-// zero, G(-n1) = G(n1)^+, so only n1 = 0 .. (b1n - 1)/2 are summed per column.
-__host__ __device__ inline bool kcol_half(const SolveTables& t) {
-  return t.hermitian && t.b1lo == -(t.b1n - 1) / 2 && t.b1n % 2 == 1 && t.b2lo == -(t.b2n - 1) / 2 && t.b2n % 2 == 1;
+__device__ __forceinline__ void kc_cp16(void* dst_smem, const void* src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// Shared-memory layout (complex double units unless noted), shared by host planning and kernel.
-struct KcolLayout {
-  size_t t1, G, GW, p2, total_cx, E_d, J_d, Y_d;
-  int nq1, tstride;
-  bool rj;  // window-contracted current (nw = 2)
-  __host__ __device__ KcolLayout(const SolveTables& t, int threads, bool half) {
-    rj = t.nw == 2;
-    nq1 = half ? (t.b1n + 1) / 2 : t.b1n;
-    tstride = threads + 2;  // twiddle rows: +2 keeps the current contraction's loads conflict-free
-    const size_t nmat = 1 + t.nax, nw2 = t.nw2, pts = t.kmode ? 2 * kRing + 1 : kRing;
-    size_t p = 0;
-    t1 = p;
-    p += (size_t)(nq1 + 4) * tstride;            // per-thread row twiddles: box rows, window rows
-    G = p;
-    p += pts * nq1 * nmat * nw2;                 // column sums of the chunk's points
-    GW = p;
-    p += (t.kmode ? 1 : kRing) * 4 * (size_t)t.nj * nw2;  // window column sums (constant: k-space solver)
-    p2 = p;
-    p += pts * (size_t)(t.b2n + 4);              // column factors of each point
-    total_cx = p;
-    E_d = 0;
-    J_d = kRing * 9;
-    Y_d = J_d + (rj ? (size_t)kRJ * (threads / 32) * 32 : (size_t)kRing * (threads / 32) * 2 * 3);
-  }
-  __host__ __device__ size_t bytes(int threads) const {
-    const size_t yd = rj ? (size_t)(threads / 32) * 4 * kYS : 0;
-    return total_cx * sizeof(double2) + (Y_d + yd) * sizeof(double);
-  }
+// The column tables in global scratch, in doubles.  A table: T0 of (D, o.x, o.y, -), then per n1 = 1..Q the
+// pairs (A, B) of each.  A step's record: real-space solver the tables at t and t + dt and the window
+// coefficients [4 state values][nj][4 rows] complex; k-space solver the tables at t + dt/2 and t + dt, with the
+// chunk's first table and the (constant) coefficients in a block per column after all records.
+// (Room for kNj current axes: models in the plane have two.)
+constexpr int kNj = 2;
+template <int Q, bool KM>
+struct Tables {
+  static constexpr int TBL = 4 + 6 * Q;
+  static constexpr int W2 = 2 * Q + 1;  // cells of a box row (narrower boxes padded with zeros)
+  static constexpr int COEF = 32 * kNj, REC = 2 * TBL + (KM ? 0 : COEF), COL = KM ? TBL + COEF : 0;
 };
 
-// HALF: the box sums run over n1 >= 0 with G(-n1) = G(n1)^+.  Per point, box row q = n1 and matrix
-// the column sums are stored as: q = 0, G(0) in slots (G00, G11, G01, G10); q > 0, (2 G00, 2 G11,
-// G01 + conj(G10), G01 - conj(G10)), so that with t = e^{-2 pi i m1 n1 / N1} = a + ib the pair
-// t G(n1) + conj(t) G(n1)^+ adds 2 Re(t G_ii) on the diagonal and a S + i b D to the upper element.
-template <int NW, int NAXc, int NJc, bool KM, bool HALF>
-__global__ void __maxnreg__(168) propagate_kcol_kernel(SolveTables t, GroupTables gt, int R,
-                                                                         int vctas, double2* rho, double2* Jpart) {
-  constexpr int NW2 = NW * NW;
-  // Window-contracted current (nw = 2): J_a = sum_{w1,e} GW_a,e(w1) R(w1, e) with
-  // R(w1, e) = sum_k tw1(k, w1) conj(rho_e(k)), the same sum as sum_k Tr(W_a(k) rho(k)^*) in another
-  // order.  Each step a warp stages its 32 k-points' state (rho00, rho11, rho01) in shared memory and
-  // lane (h, w1, c) sums tw1(k, w1) (held in registers for the tile) times state value c over the
-  // k-points of lane half h (both parts of tw1); every kRJ steps the CTA adds the warps' sums and
-  // contracts them with the column's window sums.
-  constexpr bool RJ = NW == 2;  // (the k-space solver's window sums GW are the same for every step)
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int nax = NAXc ? NAXc : t.nax, nj = NJc ? NJc : t.nj, nmat = 1 + nax;
-  const int b1n = t.b1n, b2n = t.b2n, npw = 2 * t.np + 1;
-  const int nthr = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = nthr >> 5;
-  const KcolLayout L(t, nthr, HALF);
-  const int nq1 = L.nq1, q1s = b1n - nq1, ts = L.tstride;
-  double2* sm = reinterpret_cast<double2*>(smraw);
-  double2* sT1 = sm + L.t1;
-  double2* sG = sm + L.G;
-  double2* sGW = sm + L.GW;
-  double2* sp2 = sm + L.p2;
-  double* sE = reinterpret_cast<double*>(sm + L.total_cx) + L.E_d;
-  double* sJ = reinterpret_cast<double*>(sm + L.total_cx) + L.J_d;
-  double* sY = reinterpret_cast<double*>(sm + L.total_cx) + L.Y_d + (size_t)warp * 4 * kYS;
-  const double2* X = gt.Xbox64;  // [nmat][b1n][b2n][NW2]
-  const double2* V = gt.Xwin64;  // [nj][4][4][NW2]
-  const double2* P = gt.P64;     // [points][2][npw]
-  const int ppr = KM ? 2 : 1, cstride = b2n + 4;
-  const double dt = t.dt;
-  const double prefac = 0.1666666666666 * dt;
-  const int rows = t.row1 - t.row0, tpc = (rows + R - 1) / R, ntiles = t.N2 * tpc;
-
-  double hd[NW], rd[3][NW];
-  double2 hu[NW2], ru[3][NW2], w[3][NW2];
-  // Box sums of chunk point pt (Hermitian parts: diagonal real, upper triangle complex).
-  auto box_sums = [&](int pt) {
-    if constexpr (HALF) {
-      const double2* g0 = sG + (size_t)pt * nq1 * nmat * NW2;  // n1 = 0
+// One warp: column m2, points l0 .. l0 + kTabPts - 1 of the steps [step0, step1).  Real-space solver: a point per
+// step; k-space solver: points 2 step0 + 1, ... (two per step), and the first group's extra point 2 step0.
+template <int Q, bool KM>
+struct TabSmem {
+  static constexpr int W2 = 2 * Q + 1, NP = kTabPts + (KM ? 1 : 0);
+  double2 p2[NP][W2 + 4];       // column factors: box cells n2 = -Q..Q, window cells -2..1
+  double2 p1[NP][Q + 5];        // row factors: n1 = 0..Q, window rows -2..1
+  double2 xc[4][Q + 1][3][W2];  // X00 - X11, X01, X10
+  double2 tw2[W2 + 4];
+  double es[KM ? kTabPts / 2 + 1 : kTabPts][9];
+};
+template <int Q, bool KM>
+__device__ __forceinline__ void column_tables(const SolveTables& t, const GroupTables& gt, int step0, int step1, int m2,
+                                              int l0, int chunk, double* out, TabSmem<Q, KM>& S) {
+  using TT = Tables<Q, KM>;
+  constexpr int TBL = TT::TBL, W2 = TT::W2;
+  const int lane = threadIdx.x & 31, nmat = 1 + t.nax, nj = t.nj;
+  const int half = (t.b1n - 1) / 2, npw = 2 * t.np + 1;
+  const int steps = step1 - step0, npts = KM ? 2 * steps : steps, ns = min(kTabPts, npts - l0);
+  const int first = KM && l0 == 0 ? 1 : 0, np = ns + first;
+  const double2 zero = make_double2(0.0, 0.0);
+  // local point l: l < first: the chunk's first point; else point l0 + l - first
+  auto row_of = [&](int l) { return KM ? (l < first ? 2 * step0 : 2 * step0 + 1 + l0 + l - first) : step0 + l0 + l; };
+  // (the steps' field samples of the group)
+  const int st0 = KM ? l0 >> 1 : l0, nst = KM ? (ns + 1) >> 1 : ns;
+  for (int idx = lane; idx < nst * 9; idx += 32) S.es[idx / 9][idx % 9] = t.es[(size_t)(step0 + st0) * 9 + idx];
+  if (lane < W2 + 4) S.tw2[lane] = t.T2[kc_wrap(m2 * (lane < W2 ? lane - Q : lane - W2 - 2), t.N2)];
+  for (int idx = lane; idx < nmat * (Q + 1) * W2; idx += 32) {
+    const int n2 = idx % W2 - Q, q = (idx / W2) % (Q + 1), mat = idx / (W2 * (Q + 1));
+    const bool on = q <= half && n2 >= t.b2lo && n2 <= -t.b2lo;
+    const double2* x = gt.Xbox64 + (on ? ((size_t)(mat * t.b1n + half + q) * t.b2n + n2 - t.b2lo) * 4 : 0);
+    const double2 x0 = x[0], x1 = x[1], x2 = x[2], x3 = x[3];
+    S.xc[mat][q][0][n2 + Q] = on ? make_double2(x0.x - x3.x, x0.y - x3.y) : zero;
+    S.xc[mat][q][1][n2 + Q] = on ? x1 : zero;
+    S.xc[mat][q][2][n2 + Q] = on ? x2 : zero;
+  }
+  const int clampq = min(Q, t.np);
+  for (int idx = lane; idx < np * (Q + 5); idx += 32) {
+    const int l = idx / (Q + 5), q = idx % (Q + 5);
+    const double2* P = gt.P64 + (size_t)row_of(l) * 2 * npw + t.np;
+    S.p1[l][q] = q <= Q ? P[min(q, clampq)] : P[q - Q - 3];
+  }
+  __syncwarp();
+  for (int idx = lane; idx < np * (W2 + 4); idx += 32) {
+    const int l = idx / (W2 + 4), q = idx % (W2 + 4), n2 = q < W2 ? q - Q : q - W2 - 2;
+    const double2* P = gt.P64 + (size_t)row_of(l) * 2 * npw + npw + t.np;
+    S.p2[l][q] = (KM && q >= W2) ? S.tw2[q] : kc_mul(S.tw2[q], P[max(-clampq, min(clampq, n2))]);
+  }
+  __syncwarp();
+  double* base = out + (size_t)m2 * chunk * TT::REC;
+  double* colb = out + (size_t)t.N2 * chunk * TT::REC + (size_t)m2 * TT::COL;
+  // Items (point, row n1, D or o).
+  for (int idx = lane; idx < np * (Q + 1) * 2; idx += 32) {
+    const int l = idx % np, qk = idx / np, q = qk >> 1, kind = qk & 1;
+    const int pt = l0 + l - first;  // point in the chunk; its step and field samples
+    const int st = KM ? pt >> 1 : pt;
+    const double* es = S.es[l < first ? 0 : st - st0];
+    const int e0 = KM ? (l < first ? 0 : ((pt & 1) ? 6 : 3)) : 0, e1 = 6;
+    double2 a0 = zero, a1 = zero, b0 = zero, b1 = zero;  // first and second sample: D or G01, and G10
+    for (int mat = 0; mat < nmat; ++mat) {
+      const int ax = mat == 0 ? 0 : (mat == 1 ? t.ax_id[0] : (mat == 2 ? t.ax_id[1] : t.ax_id[2]));
+      const double f0 = mat ? es[e0 + ax] : 1.0, f1 = mat ? es[e1 + ax] : 1.0;
+      double2 u = zero, h = zero;
 #pragma unroll
-      for (int i = 0; i < NW; ++i) {
-        hd[i] = g0[i].x;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) rd[a][i] = a < nax ? g0[(1 + a) * NW2 + i].x : 0.0;
+      for (int n = 0; n < W2; ++n) {
+        u = kc_fma(S.p2[l][n], S.xc[mat][q][kind][n], u);
+        if (kind) h = kc_fma(S.p2[l][n], S.xc[mat][q][2][n], h);
       }
-      if constexpr (NW == 2) {
-        hu[1] = g0[2];
+      u = kc_mul(S.p1[l][q], u);
+      h = kc_mul(S.p1[l][q], h);
+      a0 = make_double2(fma(f0, u.x, a0.x), fma(f0, u.y, a0.y));
+      b0 = make_double2(fma(f0, h.x, b0.x), fma(f0, h.y, b0.y));
+      a1 = make_double2(fma(f1, u.x, a1.x), fma(f1, u.y, a1.y));
+      b1 = make_double2(fma(f1, h.x, b1.x), fma(f1, h.y, b1.y));
+    }
 #pragma unroll
-        for (int a = 0; a < 3; ++a) ru[a][1] = a < nax ? g0[(1 + a) * NW2 + 2] : make_double2(0.0, 0.0);
+    for (int f = 0; f < (KM ? 1 : 2); ++f) {
+      const double2 a = f ? a1 : a0, b = f ? b1 : b0;
+      double* d = l < first ? colb : base + (size_t)st * TT::REC + (KM ? (pt & 1) : f) * TBL;
+      if (q == 0) {
+        if (kind == 0)
+          d[0] = a.x;
+        else
+          d[1] = a.x, d[2] = a.y;
+      } else {
+        double2* dq = reinterpret_cast<double2*>(d + 4 + 6 * (q - 1));
+        if (kind == 0) {
+          dq[0] = make_double2(2.0 * a.x, -2.0 * a.y);
+        } else {  // S = G01 + conj G10, D = G01 - conj G10
+          dq[1] = make_double2(a.x + b.x, -(a.y + b.y));
+          dq[2] = make_double2(a.y - b.y, a.x - b.x);
+        }
       }
+    }
+  }
+  // Window coefficients [value][axis][row] of rho00, rho11, Re rho01 (V01 + V10) and Im rho01 (-i (V01 - V10)), a lane
+  // each.
+  const int per = 16 * nj;
+  const int nwp = KM ? first : ns;
+  for (int c = lane; c < per; c += 32) {
+    const int w1 = c & 3, a = (c >> 2) % nj, vv = (c >> 2) / nj;
+    double2 vc[4];
+#pragma unroll
+    for (int w2 = 0; w2 < 4; ++w2) {
+      const double2* x = gt.Xwin64 + (size_t)(a * 4 + w1) * 16 + 4 * w2;
+      const double2 x0 = x[0], x1 = x[1], x2 = x[2], x3 = x[3];
+      vc[w2] = vv == 0   ? x0
+               : vv == 1 ? x3
+               : vv == 2 ? make_double2(x1.x + x2.x, x1.y + x2.y)
+                         : make_double2(x1.y - x2.y, x2.x - x1.x);
+    }
 #pragma unroll 2
-      for (int q = 1; q < nq1; ++q) {
-        const double2 tw = sT1[q * ts + tid];
-        const double2* g = g0 + (size_t)q * nmat * NW2;
+    for (int l = 0; l < nwp; ++l) {
+      double2 acc = zero;
 #pragma unroll
-        for (int i = 0; i < NW; ++i) hd[i] = fma(tw.x, g[i].x, fma(-tw.y, g[i].y, hd[i]));
-        if constexpr (NW == 2) {
-          const double2 S = g[2], D = g[3];
-          hu[1].x = fma(tw.x, S.x, fma(-tw.y, D.y, hu[1].x));
-          hu[1].y = fma(tw.x, S.y, fma(tw.y, D.x, hu[1].y));
-        }
+      for (int w2 = 0; w2 < 4; ++w2) acc = kc_fma(S.p2[l][W2 + w2], vc[w2], acc);
+      if (!KM) acc = kc_mul(S.p1[l][Q + 1 + w1], acc);
+      double* d = KM ? colb + TBL : base + (size_t)(l0 + l) * TT::REC + 2 * TBL;
+      reinterpret_cast<double2*>(d)[c] = acc;
+    }
+  }
+}
+
+template <int Q, bool KM>
+struct PropSmem {
+  using TT = Tables<Q, KM>;
+  static constexpr int YS = 34;  // row stride of the staged states, 2 mod 16 doubles: the eight rows of one load
+                                 // phase fall in distinct banks
+  double rb[3][kIv][TT::REC];    // records: the previous interval's (coefficients), this one's, the next one's
+  double cb[KM ? TT::COL : 2];   // the column's block
+  double y[2][4][2 * kIv][YS];   // row class 2 (value & 1) + (difference), row 2 step + value / 2
+};
+
+struct KcolArgs {
+  SolveTables t;      // steps [step0, step1) to propagate
+  GroupTables gt;
+  const double* cur;  // their tables
+  double* next;       // tables of [next0, next1), formed by the CTAs from nprop on
+  int next0, next1, chunk, R, vctas, nprop;
+  double2 *rho, *Jpart;
+};
+
+// SPLIT: warp 0 propagates, warp 1 forms the current; otherwise one warp does both.
+template <int Q, bool KM, bool SPLIT>
+__device__ __forceinline__ void propagate_tile(const KcolArgs& A, int v, int tile, PropSmem<Q, KM>& S) {
+  using TT = Tables<Q, KM>;
+  constexpr int TBL = TT::TBL;
+  const SolveTables& t = A.t;
+  const int lane = threadIdx.x & 31, nj = t.nj, hN = t.N1 / 2;
+  const bool steps = !SPLIT || threadIdx.x < 32, sums = !SPLIT || threadIdx.x >= 32;
+  auto sync = [] {
+    if (SPLIT)
+      __syncthreads();
+    else
+      __syncwarp();
+  };
+  const int step0 = t.step0, step1 = t.step1, nint = (step1 - step0 + kIv - 1) / kIv;
+  const double dt = t.dt, prefac = 0.1666666666666 * dt;
+  const int pairs = min(t.row1 - t.row0, hN), tpc = (pairs + A.R - 1) / A.R;
+  const int m2 = tile / tpc, i0 = (tile % tpc) * A.R, m10 = t.row0 + i0;
+  const int nown = min(A.R, pairs - i0);
+
+  const double* recs = A.cur + (size_t)m2 * A.chunk * TT::REC;
+  auto fetch = [&](int iv) {  // records of interval iv into buffer iv % 3
+    const int n = min(kIv, step1 - step0 - iv * kIv) * TT::REC / 2;
+    double* dst = &S.rb[iv % 3][0][0];
+    const double* src = recs + (size_t)iv * kIv * TT::REC;
+    if (n == kIv * TT::REC / 2) {
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (a < nax) {
-            const double2* ga = g + (1 + a) * NW2;
-#pragma unroll
-            for (int i = 0; i < NW; ++i) rd[a][i] = fma(tw.x, ga[i].x, fma(-tw.y, ga[i].y, rd[a][i]));
-            if constexpr (NW == 2) {
-              const double2 S = ga[2], D = ga[3];
-              ru[a][1].x = fma(tw.x, S.x, fma(-tw.y, D.y, ru[a][1].x));
-              ru[a][1].y = fma(tw.x, S.y, fma(tw.y, D.x, ru[a][1].y));
-            }
-          }
-      }
+      for (int q = 0; q < (kIv * TT::REC / 2 + 31) / 32; ++q)
+        if (q * 32 + lane < kIv * TT::REC / 2) kc_cp16(dst + 2 * (q * 32 + lane), src + 2 * (q * 32 + lane));
     } else {
+      for (int idx = lane; idx < n; idx += 32) kc_cp16(dst + 2 * idx, src + 2 * idx);
+    }
+  };
+  sync();  // the previous tile's readers are done
+  if (sums) fetch(0);
+  if (KM && sums) {
+    const double* src = A.cur + (size_t)t.N2 * A.chunk * TT::REC + (size_t)m2 * TT::COL;
+    for (int idx = lane; idx < TT::COL / 2; idx += 32) kc_cp16(S.cb + 2 * idx, src + 2 * idx);
+  }
+  if (sums)
+    for (int idx = lane; idx < 4 * 2 * kIv * S.YS; idx += 32) (&S.y[1][0][0][0])[idx] = 0.0;  // "interval -1"
+
+  // Sums over the rows: lane = (quarter kq of the rows, step, value pair); its rows' twiddles.
+  const int kq = lane >> 3, sl = lane & 7;
+  double twr[8][4];  // cos, sin, cos 2, sin 2 of 2 pi m1 / N1
 #pragma unroll
-      for (int i = 0; i < NW; ++i) {
-        hd[i] = 0.0;
+  for (int i = 0; i < 8; ++i) {
+    const int m1 = min(m10 + kq * 8 + i, t.N1 - 1);
+    const double2 a = t.T1[m1], b = t.T1[2 * m1 < t.N1 ? 2 * m1 : 2 * m1 - t.N1];
+    twr[i][0] = a.x;
+    twr[i][1] = -a.y;
+    twr[i][2] = b.x;
+    twr[i][3] = -b.y;
+  }
+  // The lane's place in the contraction: value vv, axis ja, step sl / 2.
+  const bool hi = lane >= 16;
+  const int ja = kq & 1, jcoef = ((2 * (lane & 1) + (hi ? 1 : 0)) * nj + ja) * 4;
+  double2* Jrow = A.Jpart + ((size_t)v * t.nt + step0 + (sl >> 1)) * 3 + (ja ? t.j_id[1] : t.j_id[0]);
+  double z[2][5];
+  auto clear = [&] {
 #pragma unroll
-        for (int a = 0; a < 3; ++a) rd[a][i] = 0.0;
-      }
+    for (int i = 0; i < 5; ++i) z[0][i] = z[1][i] = 0.0;
+  };
+  // Rows 2 part, 2 part + 1 of the quarter, staged in buffer b.
+  auto sum_part = [&](int part, int b) {
 #pragma unroll
-      for (int e = 0; e < NW2; ++e) {
-        hu[e] = make_double2(0.0, 0.0);
+    for (int u = 0; u < 2; ++u) {
+      const double2 yp = *reinterpret_cast<const double2*>(&S.y[b][2 * u][sl][kq * 8 + 2 * part]);
+      const double2 ym = *reinterpret_cast<const double2*>(&S.y[b][2 * u + 1][sl][kq * 8 + 2 * part]);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) ru[a][e] = make_double2(0.0, 0.0);
-      }
-#pragma unroll 4
-      for (int q1 = 0; q1 < b1n; ++q1) {
-        const double2 tw = sT1[q1 * ts + tid];
-        const double2* g = sG + ((size_t)pt * b1n + q1) * nmat * NW2;
-#pragma unroll
-        for (int i = 0; i < NW; ++i) {
-          hd[i] = fma(tw.x, g[i * NW + i].x, fma(-tw.y, g[i * NW + i].y, hd[i]));
-#pragma unroll
-          for (int j = i + 1; j < NW; ++j) hu[i * NW + j] = kc_fma(tw, g[i * NW + j], hu[i * NW + j]);
-        }
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (a < nax) {
-            const double2* ga = g + (1 + a) * NW2;
-#pragma unroll
-            for (int i = 0; i < NW; ++i) {
-              rd[a][i] = fma(tw.x, ga[i * NW + i].x, fma(-tw.y, ga[i * NW + i].y, rd[a][i]));
-#pragma unroll
-              for (int j = i + 1; j < NW; ++j) ru[a][i * NW + j] = kc_fma(tw, ga[i * NW + j], ru[a][i * NW + j]);
-            }
-          }
+      for (int e = 0; e < 2; ++e) {
+        const double* w = twr[2 * part + e];
+        const double p = e ? yp.y : yp.x, m = e ? ym.y : ym.x;
+        z[u][0] += p;
+        z[u][1] = fma(w[0], m, z[u][1]);
+        z[u][2] = fma(w[1], m, z[u][2]);
+        z[u][3] = fma(w[2], p, z[u][3]);
+        z[u][4] = fma(w[3], p, z[u][4]);
       }
     }
   };
-  // Window velocity W_a(k) from the column sums of slot s.
-  auto window_sums = [&](int s) {
+  // Interval iv's sums over the quarters (the upper lanes keep the second value's, the lower the first's), times
+  // the coefficients, into its row of partials; iv < 0: nothing is stored.
+  auto finish = [&](int iv) {
+    double q[5];
 #pragma unroll
-    for (int e = 0; e < NW2; ++e)
-#pragma unroll
-      for (int a = 0; a < 3; ++a) w[a][e] = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int w1 = 0; w1 < 4; ++w1) {
-      const double2 tw = sT1[(nq1 + w1) * ts + tid];
-      const double2* g = sGW + ((size_t)s * 4 + w1) * nj * NW2;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        if (a < nj)
-#pragma unroll
-          for (int e = 0; e < NW2; ++e) w[a][e] = kc_fma(tw, g[a * NW2 + e], w[a][e]);
+    for (int i = 0; i < 5; ++i) {
+      const double keep = hi ? z[1][i] : z[0][i], send = hi ? z[0][i] : z[1][i];
+      q[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+      q[i] += __shfl_xor_sync(0xffffffffu, q[i], 8);
     }
-  };
-  // Column sum of point s, box row q1 (table index), matrix mat, element e, times the row factor.
-  auto column_sum = [&](int s, int q1, int mat, int e, int j0) {
-    const double2* x = X + ((size_t)(mat * b1n + q1) * b2n) * NW2 + e;
-    const double2* p2 = sp2 + s * cstride;
-    double2 acc = make_double2(0.0, 0.0);
-    for (int q2 = 0; q2 < b2n; ++q2) acc = kc_fma(p2[q2], x[(size_t)q2 * NW2], acc);
-    return kc_mul(P[(size_t)(j0 + s) * 2 * npw + t.np + t.b1lo + q1], acc);
+    const bool on = iv >= 0 && ja < nj && step0 + iv * kIv + (sl >> 1) < step1;
+    double re = 0.0, im = 0.0;
+    if (on) {
+      // rows n1 = -2, -1, 0, 1 have the sums (q3, q4), (q1, q2), (q0, 0), (q1, -q2)
+      const double2* cf = reinterpret_cast<const double2*>(KM ? S.cb + TBL : &S.rb[iv % 3][sl >> 1][2 * TBL]) + jcoef;
+      const double2 f0 = cf[0], f1 = cf[1], f2 = cf[2], f3 = cf[3];
+      re = fma(f0.x, q[3], fma(-f0.y, q[4], fma(f1.x + f3.x, q[1], fma(f3.y - f1.y, q[2], f2.x * q[0]))));
+      im = fma(f0.x, q[4], fma(f0.y, q[3], fma(f1.x - f3.x, q[2], fma(f1.y + f3.y, q[1], f2.y * q[0]))));
+    }
+    re += __shfl_xor_sync(0xffffffffu, re, 1);
+    im += __shfl_xor_sync(0xffffffffu, im, 1);
+    re += __shfl_xor_sync(0xffffffffu, re, 16);
+    im += __shfl_xor_sync(0xffffffffu, im, 16);
+    if (on && (lane & 17) == 0) {
+      double2* dst = Jrow + (ptrdiff_t)iv * kIv * 3;
+      // the virtual CTA's first tile writes its row (cleared before the launch) without reading it
+      const double2 old = tile == v ? make_double2(0.0, 0.0) : *dst;
+      *dst = make_double2(old.x + re, old.y + im);
+    }
   };
 
+  // States of the k-points (m1, m2) and (m1 + N1/2, m2), m1 = m10 + lane.
+  const bool on0 = steps && lane < nown, on1 = on0 && m10 + lane + hN < t.row1;
+  const size_t k0 = (size_t)(m10 + (on0 ? lane : 0)) * t.N2 + m2, k1 = on1 ? k0 + (size_t)hN * t.N2 : k0;
+  double r00[2] = {}, r11[2] = {}, ux[2] = {}, uy[2] = {}, twa[Q], twb[Q];
+  double hD[2] = {}, hx[2] = {}, hy[2] = {};  // k-space solver: H at the step's t, carried
+  auto get = [&](size_t k, int j) {
+    r00[j] = A.rho[k * 4].x;
+    r11[j] = A.rho[k * 4 + 3].x;
+    ux[j] = A.rho[k * 4 + 1].x;
+    uy[j] = A.rho[k * 4 + 1].y;
+  };
+  if (on0) get(k0, 0);
+  if (on1) get(k1, 1);
+  {
+    const int m1 = min(m10 + lane, t.N1 - 1);
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const double2 a = t.T1[kc_wrap((long long)m1 * (q + 1), t.N1)];
+      twa[q] = a.x;
+      twb[q] = a.y;
+    }
+  }
+  // H of both rows from one table: e the terms of even n1, o those of odd.
+  auto eval = [&](const double* tb, double (&D)[2], double (&ox)[2], double (&oy)[2]) {
+    const double2 z0 = *reinterpret_cast<const double2*>(tb);
+    double e[3] = {z0.x, z0.y, tb[2]}, o[3];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const double2 a = *reinterpret_cast<const double2*>(tb + 4 + 6 * q + 2 * i);
+        if (q == 0)
+          o[i] = fma(twa[q], a.x, twb[q] * a.y);
+        else if (q % 2 == 1)
+          e[i] = fma(twa[q], a.x, fma(twb[q], a.y, e[i]));
+        else
+          o[i] = fma(twa[q], a.x, fma(twb[q], a.y, o[i]));
+      }
+    }
+    D[0] = e[0] + o[0];
+    D[1] = e[0] - o[0];
+    ox[0] = e[1] + o[1];
+    ox[1] = e[1] - o[1];
+    oy[0] = e[2] + o[2];
+    oy[1] = e[2] - o[2];
+  };
+  // H of a step at its three points (real-space solver: [1] is twice H at t + dt/2).
+  struct Hs {
+    double D[3][2], x[3][2], y[3][2];
+  };
+  auto load = [&](const double* tb, Hs& h) {
+    if constexpr (KM) {
+      eval(tb, h.D[1], h.x[1], h.y[1]);
+      eval(tb + TBL, h.D[2], h.x[2], h.y[2]);
+    } else {
+      eval(tb, h.D[0], h.x[0], h.y[0]);
+      eval(tb + TBL, h.D[2], h.x[2], h.y[2]);
+    }
+  };
+  auto step = [&](Hs& h) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      if constexpr (KM) {
+        h.D[0][j] = hD[j];
+        h.x[0][j] = hx[j];
+        h.y[0][j] = hy[j];
+        hD[j] = h.D[2][j];
+        hx[j] = h.x[2][j];
+        hy[j] = h.y[2][j];
+      } else {
+        h.D[1][j] = h.D[0][j] + h.D[2][j];
+        h.x[1][j] = h.x[0][j] + h.x[2][j];
+        h.y[1][j] = h.y[0][j] + h.y[2][j];
+      }
+    }
+    // RK4 (src/solver.cpp:157-163): X = rho + c k~, the middle stages' k~ twice k in the real-space solver;
+    // kd = k00 / 2, k01 = (ty, -tx).
+    const double c0 = 0.5 * dt, cm = KM ? 0.5 * dt : 0.25 * dt, ce = KM ? dt : 0.5 * dt;
+    double d[2], xd[2], xx[2], xy[2], kd[2], tx[2], ty[2], sd[2], sx[2], sy[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      xd[j] = d[j] = r00[j] - r11[j];
+      xx[j] = ux[j];
+      xy[j] = uy[j];
+    }
+#pragma unroll
+    for (int st = 0; st < 4; ++st) {
+      const int p = st == 0 ? 0 : (st == 3 ? 2 : 1);
+      const double c = st == 0 ? c0 : (st == 1 ? cm : ce);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        kd[j] = h.x[p][j] * xy[j];
+        tx[j] = xd[j] * h.x[p][j];
+        ty[j] = xd[j] * h.y[p][j];
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        kd[j] = fma(h.y[p][j], xx[j], -kd[j]);
+        tx[j] = fma(h.D[p][j], xx[j], -tx[j]);
+        ty[j] = fma(h.D[p][j], xy[j], -ty[j]);
+      }
+      if (st < 3) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          xd[j] = fma(4.0 * c, kd[j], d[j]);
+          xx[j] = fma(c, ty[j], ux[j]);
+          xy[j] = fma(-c, tx[j], uy[j]);
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (st == 0) {
+          sd[j] = kd[j];
+          sx[j] = tx[j];
+          sy[j] = ty[j];
+        } else if (KM && st < 3) {
+          sd[j] = fma(2.0, kd[j], sd[j]);
+          sx[j] = fma(2.0, tx[j], sx[j]);
+          sy[j] = fma(2.0, ty[j], sy[j]);
+        } else {
+          sd[j] += kd[j];
+          sx[j] += tx[j];
+          sy[j] += ty[j];
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      r00[j] = fma(2.0 * prefac, sd[j], r00[j]);
+      r11[j] = fma(-2.0 * prefac, sd[j], r11[j]);
+      ux[j] = fma(prefac, sy[j], ux[j]);
+      uy[j] = fma(-prefac, sx[j], uy[j]);
+    }
+  };
+  // Staged for the current: sums and differences of the pair (absent rows stay zero: their state is 0 and the
+  // commutator keeps it there).
+  auto stage = [&](int s, int b) {
+    S.y[b][0][2 * s][lane] = r00[0] + r00[1];
+    S.y[b][1][2 * s][lane] = r00[0] - r00[1];
+    S.y[b][2][2 * s][lane] = r11[0] + r11[1];
+    S.y[b][3][2 * s][lane] = r11[0] - r11[1];
+    S.y[b][0][2 * s + 1][lane] = ux[0] + ux[1];
+    S.y[b][1][2 * s + 1][lane] = ux[0] - ux[1];
+    S.y[b][2][2 * s + 1][lane] = uy[0] + uy[1];
+    S.y[b][3][2 * s + 1][lane] = uy[0] - uy[1];
+  };
+  auto last_sums = [&](int iv) {
+    clear();
+#pragma unroll
+    for (int s = 0; s < kIv; ++s) sum_part(s, iv & 1);
+    finish(iv);
+  };
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  sync();
+  if (KM && steps) eval(S.cb, hD, hx, hy);
+
+  for (int iv = 0; iv < nint; ++iv) {
+    const int b = iv & 1, ns = min(kIv, step1 - step0 - iv * kIv);
+    const double(*rec)[TT::REC] = S.rb[iv % 3];
+    if (sums && iv + 1 < nint) fetch(iv + 1);
+    if (SPLIT && sums) {
+      last_sums(iv - 1);
+    } else {
+      if (!SPLIT) clear();
+      // A whole interval unrolled.  The next step's H and the previous interval's sums come before this step's
+      // stores (their loads could not pass them); neither depends on the state.
+      Hs h[2];
+      load(rec[0], h[0]);
+      if (ns == kIv) {
+#pragma unroll
+        for (int s = 0; s < kIv; ++s) {
+          if (s + 1 < kIv) load(rec[s + 1], h[(s + 1) & 1]);
+          if (!SPLIT) {
+            sum_part(s, b ^ 1);
+            if (s + 1 == kIv) finish(iv - 1);
+          }
+          step(h[s & 1]);
+          stage(s, b);
+        }
+      } else {
+        if (!SPLIT) {
+#pragma unroll
+          for (int s = 0; s < kIv; ++s) sum_part(s, b ^ 1);
+          finish(iv - 1);
+        }
+#pragma unroll 1
+        for (int s = 0; s < ns; ++s) {
+          if (s > 0) load(rec[s], h[0]);
+          step(h[0]);
+          stage(s, b);
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    sync();
+  }
+  if (sums) last_sums(nint - 1);
+  auto put = [&](size_t k, int j) {
+    A.rho[k * 4] = make_double2(r00[j], 0.0);
+    A.rho[k * 4 + 1] = make_double2(ux[j], uy[j]);
+    A.rho[k * 4 + 2] = make_double2(ux[j], -uy[j]);
+    A.rho[k * 4 + 3] = make_double2(r11[j], 0.0);
+  };
+  if (on0) put(k0, 0);
+  if (on1) put(k1, 1);
+}
+
+template <int Q, bool KM>
+union KcolSmem {
+  PropSmem<Q, KM> prop;
+  TabSmem<Q, KM> tab;
+};
+
+template <int Q, bool KM, bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 64 : 32, SPLIT ? 4 : 8) propagate_kcol_kernel(const __grid_constant__ KcolArgs A) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  KcolSmem<Q, KM>& S = *reinterpret_cast<KcolSmem<Q, KM>*>(smraw);
+  if ((int)blockIdx.x >= A.nprop) {
+    const int idx = blockIdx.x - A.nprop;
+    if (SPLIT && threadIdx.x >= 32) return;
+    column_tables<Q, KM>(A.t, A.gt, A.next0, A.next1, idx % A.t.N2, idx / A.t.N2 * kTabPts, A.chunk, A.next, S.tab);
+    return;
+  }
   // Virtual CTA v owns tiles v, v + vctas, ... and its own row of current partials.
-  for (int v = blockIdx.x; v < vctas; v += gridDim.x)
-  for (int tile = v; tile < ntiles; tile += vctas) {
-    const int m2 = tile / tpc, m1r = t.row0 + (tile % tpc) * R + tid;
-    const bool kval = tid < R && m1r < t.row1;
-    const int m1 = kval ? m1r : t.row0;
-    const size_t k = (size_t)m1 * t.N2 + m2;
-    double2 r[NW2];
-#pragma unroll
-    for (int e = 0; e < NW2; ++e) r[e] = kval ? rho[k * NW2 + e] : make_double2(0.0, 0.0);
-    for (int q = 0; q < nq1; ++q) sT1[q * ts + tid] = t.T1[kc_wrap((long long)m1 * (t.b1lo + q1s + q), t.N1)];
-    for (int q = 0; q < 4; ++q) sT1[(nq1 + q) * ts + tid] = t.T1[kc_wrap((long long)m1 * (q - 2), t.N1)];
-    // This lane's twiddles in the current contraction (RJ): tw1(k, w1) of the warp's k-points
-    // k = 4j + 2h + b (j < 8, b < 2) of lane half h, for the lane's window row w1.
-    double2 twc[RJ ? 16 : 1];
-    if constexpr (RJ) {
-      const int h = lane >> 4, w1 = (lane >> 2) & 3, m1w = t.row0 + (tile % tpc) * R + warp * 32;
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        twc[j] = t.T1[kc_wrap((long long)(m1w + 4 * (j >> 1) + 2 * h + (j & 1)) * (w1 - 2), t.N1)];
-    }
-
-    for (int ti0 = t.step0; ti0 < t.step1; ti0 += kRing) {
-      const int nsteps = min(kRing, t.step1 - ti0);
-      const int npts = KM ? 2 * nsteps + 1 : nsteps, j0 = ppr * ti0;
-      __syncthreads();  // the previous chunk's readers are done
-      // (a) column factors of each point: box n2 = b2lo + q, then window n2 = -2..1
-      for (int idx = tid; idx < npts * cstride; idx += nthr) {
-        const int s = idx / cstride, q = idx % cstride;
-        const int n2 = q < b2n ? t.b2lo + q : q - b2n - 2;
-        const double2 tw = t.T2[kc_wrap((long long)m2 * n2, t.N2)];
-        sp2[idx] = (KM && q >= b2n) ? tw : kc_mul(tw, P[((size_t)(j0 + s) * 2 + 1) * npw + t.np + n2]);
-      }
-      for (int idx = tid; idx < nsteps * 9; idx += nthr) sE[idx] = t.es[(size_t)ti0 * 9 + idx];
-      __syncthreads();
-      // (b) the column's sums G(n1) of each point, times the row factor P1(n1)
-      const int nG = npts * nq1 * nmat * NW2;
-      for (int idx = tid; idx < nG; idx += nthr) {
-        const int e = idx % NW2;
-        int rest = idx / NW2;
-        const int mat = rest % nmat;
-        rest /= nmat;
-        const int q = rest % nq1, s = rest / nq1;
-        double2 val;
-        if constexpr (HALF) {
-          // slot e of the stored form (see above); element index i * NW + j
-          if (q == 0 || e < NW) {
-            const int src = NW == 2 ? (e == 0 ? 0 : e == 1 ? 3 : e == 2 ? 1 : 2) : 0;
-            val = column_sum(s, q1s + q, mat, src, j0);
-            if (q > 0) val = make_double2(2.0 * val.x, 2.0 * val.y);
-          } else {
-            const double2 g01 = column_sum(s, q1s + q, mat, 1, j0), g10 = column_sum(s, q1s + q, mat, 2, j0);
-            val = e == 2 ? make_double2(g01.x + g10.x, g01.y - g10.y) : make_double2(g01.x - g10.x, g01.y + g10.y);
-          }
-        } else {
-          val = column_sum(s, q, mat, e, j0);
-        }
-        sG[idx] = val;
-      }
-      const bool win_now = !KM || ti0 == t.step0;  // the k-space solver's window sums are constant
-      if (win_now) {
-        const int nW = (KM ? 1 : nsteps) * 4 * nj * NW2;
-        for (int idx = tid; idx < nW; idx += nthr) {
-          const int e = idx % NW2;
-          int rest = idx / NW2;
-          const int a = rest % nj;
-          rest /= nj;
-          const int w1 = rest % 4, s = rest / 4;
-          const double2* vv = V + ((size_t)(a * 4 + w1) * 4) * NW2 + e;
-          const double2* p2 = sp2 + s * cstride + b2n;
-          double2 acc = make_double2(0.0, 0.0);
-#pragma unroll
-          for (int w2 = 0; w2 < 4; ++w2) acc = kc_fma(p2[w2], vv[(size_t)w2 * NW2], acc);
-          sGW[idx] = KM ? acc : kc_mul(P[(size_t)(j0 + s) * 2 * npw + t.np + (w1 - 2)], acc);
-        }
-      }
-      __syncthreads();
-      if (KM && !RJ && ti0 == t.step0) window_sums(0);
-
-      for (int s = 0; s < nsteps; ++s) {
-        if (!KM) {
-          box_sums(s);
-          if (!RJ) window_sums(s);
-        } else if (s == 0) {
-          box_sums(0);  // point t of the chunk's first step; later steps carry it from stage 4
-        }
-        if constexpr (NW == 2) {
-          herm2_rk4_step<NAXc>(r, hd, hu, rd, ru, nax, t.ax_id, sE + s * 9, dt, prefac, [&](int f) {
-            if (KM) box_sums(2 * s + f);  // the k-space solver's points t + dt/2, t + dt
-          });
-        } else {
-          // One orbital: k = -i (h x - conj(h x)) = 2 h Im(x) is real, so Im(x) = Im(rho) in every stage
-          // (src/solver.cpp:157-163: fields at t, t+dt/2, t+dt/2, t+dt).
-          double sk = 0.0;
-#pragma unroll
-          for (int st = 0; st < 4; ++st) {
-            const int f = st == 0 ? 0 : (st == 3 ? 2 : 1);
-            const double* es = sE + s * 9 + f * 3;
-            if (KM && (st == 1 || st == 3)) box_sums(2 * s + f);  // points t + dt/2, t + dt
-            double h = hd[0];
-#pragma unroll
-            for (int a = 0; a < 3; ++a)
-              if (a < nax) h = fma(es[t.ax_id[a]], rd[a][0], h);
-            const double kx = 2.0 * (h * r[0].y);
-            sk = st == 0 ? kx : fma(st == 3 ? 1.0 : 2.0, kx, sk);
-          }
-          r[0].x = fma(prefac, sk, r[0].x);
-        }
-
-        // Current partials.
-        if constexpr (RJ) {
-          __syncwarp();  // the previous step's readers of this warp's staging rows are done
-          sY[lane] = kval ? r[0].x : 0.0;
-          sY[kYS + lane] = kval ? r[3].x : 0.0;
-          sY[2 * kYS + lane] = kval ? r[1].x : 0.0;
-          sY[3 * kYS + lane] = kval ? r[1].y : 0.0;
-          __syncwarp();
-          const int h = lane >> 4, w1 = (lane >> 2) & 3, c = lane & 3;
-          const double* yp = sY + c * kYS + 2 * h;
-          double bx0 = 0.0, by0 = 0.0, bx1 = 0.0, by1 = 0.0;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const double2 y = *reinterpret_cast<const double2*>(yp + 4 * j);  // k = 4j + 2h, 4j + 2h + 1
-            bx0 = fma(twc[2 * j].x, y.x, bx0);
-            by0 = fma(twc[2 * j].y, y.x, by0);
-            bx1 = fma(twc[2 * j + 1].x, y.y, bx1);
-            by1 = fma(twc[2 * j + 1].y, y.y, by1);
-          }
-          double bx = bx0 + bx1, by = by0 + by1;
-          bx += __shfl_xor_sync(0xffffffffu, bx, 16);
-          by += __shfl_xor_sync(0xffffffffu, by, 16);
-          if (h == 0)
-            reinterpret_cast<double2*>(sJ)[((s % kRJ) * nwarps + warp) * 16 + w1 * 4 + c] = make_double2(bx, by);
-          if (s % kRJ == kRJ - 1 || s == nsteps - 1) {
-            const int s0f = s - s % kRJ, ns = s - s0f + 1;
-            __syncthreads();
-            // Warps' partials, in warp order, into warp 0's slot.
-            for (int idx = tid; idx < ns * 32; idx += nthr) {
-              const int ss = idx >> 5, l = idx & 31;
-              double acc = 0.0;
-              for (int q = 0; q < nwarps; ++q) acc += sJ[(ss * nwarps + q) * 32 + l];
-              sJ[(ss * nwarps) * 32 + l] = acc;
-            }
-            __syncthreads();
-            for (int idx = tid; idx < ns * nj; idx += nthr) {
-              const int ss = idx / nj, a = idx % nj;
-              const double* B = sJ + (ss * nwarps) * 32;  // B[(w1 * 4 + c) * 2 + part]
-              double re = 0.0, im = 0.0;
-#pragma unroll
-              for (int w1 = 0; w1 < 4; ++w1) {
-                const double2* g = sGW + ((size_t)((KM ? 0 : s0f + ss) * 4 + w1) * nj + a) * NW2;
-                const double* b = B + w1 * 8;
-                // R(w1, e) = sum_k tw1 conj(rho_e): e = 00, 01, 10, 11 from the state values' sums
-                const double2 Rv[4] = {make_double2(b[0], b[1]), make_double2(b[4] + b[7], b[5] - b[6]),
-                                       make_double2(b[4] - b[7], b[5] + b[6]), make_double2(b[2], b[3])};
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  re = fma(g[e].x, Rv[e].x, fma(-g[e].y, Rv[e].y, re));
-                  im = fma(g[e].x, Rv[e].y, fma(g[e].y, Rv[e].x, im));
-                }
-              }
-              double2* dst = Jpart + ((size_t)v * t.nt + ti0 + s0f + ss) * 3 + t.j_id[a];
-              // the virtual CTA's first tile writes its row (cleared before the launch) without reading it
-              const double2 old = tile == v ? make_double2(0.0, 0.0) : *dst;
-              *dst = make_double2(old.x + re, old.y + im);
-            }
-            __syncthreads();  // the slots are rewritten by the next steps
-          }
-        } else {
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          if (a < nj) {
-            double re = 0.0, im = 0.0;
-            if (kval) {
-#pragma unroll
-              for (int e = 0; e < NW2; ++e) {
-                re = fma(w[a][e].x, r[e].x, fma(w[a][e].y, r[e].y, re));
-                im = fma(w[a][e].y, r[e].x, fma(-w[a][e].x, r[e].y, im));
-              }
-            }
-            re = kc_warp_sum(re);
-            im = kc_warp_sum(im);
-            if (lane == 0) {
-              sJ[(s * nwarps + warp) * 2 * nj + 2 * a] = re;
-              sJ[(s * nwarps + warp) * 2 * nj + 2 * a + 1] = im;
-            }
-          }
-        }
-      }
-      if constexpr (RJ) continue;  // flushed inside the step loop
-      __syncthreads();
-      // Add the chunk's per-warp partials into this virtual CTA's row.
-      for (int idx = tid; idx < nsteps * nj; idx += nthr) {
-        const int s = idx / nj, a = idx % nj;
-        double re = 0.0, im = 0.0;
-        for (int q = 0; q < nwarps; ++q) {
-          re += sJ[(s * nwarps + q) * 2 * nj + 2 * a];
-          im += sJ[(s * nwarps + q) * 2 * nj + 2 * a + 1];
-        }
-        double2* dst = Jpart + ((size_t)v * t.nt + ti0 + s) * 3 + t.j_id[a];
-        const double2 old = tile == v ? make_double2(0.0, 0.0) : *dst;
-        *dst = make_double2(old.x + re, old.y + im);
-      }
-    }
-    if (kval) {
-#pragma unroll
-      for (int e = 0; e < NW2; ++e) rho[k * NW2 + e] = r[e];
-    }
-  }
+  const int pairs = min(A.t.row1 - A.t.row0, A.t.N1 / 2), ntiles = A.t.N2 * ((pairs + A.R - 1) / A.R);
+  for (int v = blockIdx.x; v < A.vctas; v += A.nprop)
+    for (int tile = v; tile < ntiles; tile += A.vctas) propagate_tile<Q, KM, SPLIT>(A, v, tile, S.prop);
 }
 
-using KcolKernel = void (*)(SolveTables, GroupTables, int, int, double2*, double2*);
-
-// Halving applies unless HHG_KCOL_FULLBOX=1 (both forms are tested against the goldens).
-bool kcol_use_half(const SolveTables& t) {
-  const char* e = std::getenv("HHG_KCOL_FULLBOX");
-  return kcol_half(t) && !(e && e[0] == '1');
+using KcolKernel = void (*)(const KcolArgs);
+struct Form {
+  KcolKernel kern[2];     // one warp per tile, two
+  size_t smem, rec, col;  // bytes; doubles per step and column of the tables
+};
+template <int Q, bool KM>
+constexpr Form form_t() {
+  return {{propagate_kcol_kernel<Q, KM, false>, propagate_kcol_kernel<Q, KM, true>}, sizeof(KcolSmem<Q, KM>), Tables<Q, KM>::REC, Tables<Q, KM>::COL};
 }
-
-template <bool KM, bool HALF>
-KcolKernel kcol_kernel_t(const SolveTables& t) {
-  if (t.nw == 2 && t.nj == 2) {
-    if (t.nax == 1) return propagate_kcol_kernel<2, 1, 2, KM, HALF>;
-    if (t.nax == 2) return propagate_kcol_kernel<2, 2, 2, KM, HALF>;
-  }
-  return t.nw == 1 ? propagate_kcol_kernel<1, 0, 0, KM, HALF> : propagate_kcol_kernel<2, 0, 0, KM, HALF>;
+Form form_of(const SolveTables& t) {
+  if (std::max(t.b1n, t.b2n) > 5) return t.kmode ? form_t<3, true>() : form_t<3, false>();
+  return t.kmode ? form_t<2, true>() : form_t<2, false>();
 }
-KcolKernel kcol_kernel_for(const SolveTables& t, bool half) {
-  if (t.kmode) return half ? kcol_kernel_t<true, true>(t) : kcol_kernel_t<true, false>(t);
-  return half ? kcol_kernel_t<false, true>(t) : kcol_kernel_t<false, false>(t);
-}
+constexpr int kPairVariant = 2;  // LaunchShape::variant of this kernel (0, 1: sbe_kcol_any.cu)
 
 }  // namespace
 
 bool plan_kcol(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem_max, int parts_hint) {
-  if (t.nw > 2 || !t.hermitian) return false;
-  const int rows = t.row1 - t.row0;
-  // Rows per tile: equal parts of at most 128 rows (measured on the 200x200 grid: 100-row tiles,
-  // four resident CTAs per SM, beat whole 200-row columns by 16 % and 50-row tiles by 30 %).
-  int parts = (rows + 127) / 128;
-  if (parts_hint > 0) parts = std::max((rows + kKcolMaxThreads - 1) / kKcolMaxThreads, parts_hint);
-  if (const char* e = std::getenv("HHG_KCOL_PARTS")) parts = std::max(parts, std::atoi(e));  // tuning override
-  const int R = (rows + parts - 1) / parts;
-  const int threads = (R + 31) / 32 * 32;
-  const long ntiles = (long)t.N2 * ((rows + R - 1) / R);
-  const bool half = kcol_use_half(t);
-  const KcolLayout L(t, threads, half);
-  const size_t smem = L.bytes(threads);
-  if (smem > smem_max || threads > kKcolMaxThreads) return false;
-  KcolKernel kern = kcol_kernel_for(t, half);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const char* full = std::getenv("HHG_KCOL_FULLBOX");
+  const bool symmetric = t.b1n % 2 == 1 && t.b1lo == -(t.b1n - 1) / 2 && t.b2n % 2 == 1 && t.b2lo == -(t.b2n - 1) / 2;
+  if (t.nw != 2 || !t.hermitian || !symmetric || t.nj > kNj || t.b1n > 7 || t.b2n > 7 || (full && full[0] == '1'))
+    return plan_kcol_any(t, sm_count, out, smem_max, parts_hint);
+  // Tiles of equal parts of a column of at most 32 pairs.
+  const int pairs = std::min(t.row1 - t.row0, t.N1 / 2), least = (pairs + 31) / 32;
+  int parts = std::max(least, parts_hint);
+  if (const char* e = std::getenv("HHG_KCOL_PARTS")) parts = std::max(least, std::atoi(e));  // tuning override
+  const int R = (pairs + parts - 1) / parts;
+  const long ntiles = (long)t.N2 * ((pairs + R - 1) / R);
+  const Form f = form_of(t);
+  // Two warps a tile up to 1.5 tiles an SM: 1024 steps of a 20 x 20 grid (20 tiles) 0.27 ms against 0.38 with one,
+  // 100 x 100 (200 tiles) 0.31 against 0.39; beyond, the second warps' registers and barriers cost more than they
+  // hide: 120 x 120 (240 tiles) 0.45 against 0.40, 200 x 200 (800 tiles, 4096 steps) 2.90 against 2.60.
+  const int warps = 2 * ntiles <= 3 * sm_count ? 2 : 1;
+  const KcolKernel kern = f.kern[warps - 1];
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
   int occ = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem);
-  if (occ < 1) return false;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * warps, f.smem);
+  if (occ < 1) return plan_kcol_any(t, sm_count, out, smem_max, parts_hint);
   const long slots = (long)occ * sm_count;
   out->kernel = 3;
   out->kmode = t.kmode;
-  out->k_per_cta = R;
+  out->k_per_cta = 2 * R;
   out->group = 1;
-  out->threads = threads;
+  out->threads = 32 * warps;
   out->ntiles = (int)ntiles;
   out->ctas = (int)(ntiles < slots ? ntiles : slots);
   out->vctas = out->ctas;
   out->box_sm = out->win_sm = 0;
   out->ept = 1;
-  out->variant = half ? 1 : 0;
-  out->smem = smem;
+  out->variant = kPairVariant;
+  out->smem = f.smem;
+  out->pre_chunk = std::min(kKcolChunk, t.nt);
+  out->pre_bytes = 2 * 8 * (size_t)t.N2 * (out->pre_chunk * f.rec + f.col);
   return true;
 }
 
-void launch_kcol(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
-                 cudaStream_t stream) {
-  KcolKernel kern = kcol_kernel_for(t, s.variant == 1);
+int launch_kcol(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
+                cudaStream_t stream) {
+  if (s.variant != kPairVariant) {
+    launch_kcol_any(t, gt, s, rho, Jpart, stream);
+    return 1;
+  }
+  if (!gt.pre || s.pre_chunk <= 0)
+    throw std::runtime_error("column-tile launch: needs its table scratch (GroupTables::pre)");
+  const Form f = form_of(t);
+  const KcolKernel kern = f.kern[s.threads / 32 - 1];
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
-  kern<<<s.ctas, s.threads, s.smem, stream>>>(t, gt, s.k_per_cta, s.vctas, rho, Jpart);
+  double* tables[2] = {static_cast<double*>(gt.pre), static_cast<double*>(gt.pre) + (size_t)t.N2 * (s.pre_chunk * f.rec + f.col)};
+  KcolArgs a{};
+  a.t = t;
+  a.gt = gt;
+  a.chunk = s.pre_chunk;
+  a.R = s.k_per_cta / 2;
+  a.vctas = s.vctas;
+  a.rho = rho;
+  a.Jpart = Jpart;
+  int launches = 0;
+  // The first launch forms the first chunk's tables only; each later one propagates a chunk and forms the next's.
+  for (int c0 = t.step0 - s.pre_chunk; c0 < t.step1; c0 += s.pre_chunk) {
+    a.next0 = std::min(c0 + s.pre_chunk, t.step1);
+    a.next1 = std::min(a.next0 + s.pre_chunk, t.step1);
+    a.next = tables[launches & 1];
+    a.cur = tables[(launches + 1) & 1];
+    a.nprop = launches == 0 ? 0 : s.ctas;
+    a.t.step0 = c0;
+    a.t.step1 = a.next0;
+    const int pts = (t.kmode ? 2 : 1) * (a.next1 - a.next0), groups = (pts + kTabPts - 1) / kTabPts;
+    kern<<<a.nprop + groups * t.N2, s.threads, s.smem, stream>>>(a);
+    ++launches;
+  }
+  return launches;
 }
 
 }  // namespace hhg
