@@ -29,7 +29,7 @@
 //    Re M_ij = a0 G0.x + sum_{n1 > 0} (a S.x - b D.y),  Im M_ij = a0 G0.y + sum (a S.y + b D.x),
 //    S = G_ij + conj G_ji,  D = G_ij - conj G_ji,
 // so the CTA's k-points (rows) times the real and imaginary parts of the elements i <= j (columns) take
-// 2 k-steps [a0 a1 a2 a3 | b1 b2 b3 0] per 8 x 8 tile.  dfrag_sums_kernel forms the S and D columns of a
+// 2 k-steps [a0 0 a1 b1 | a2 b2 a3 b3] per 8 x 8 tile.  dfrag_sums_kernel forms the S and D columns of a
 // chunk of 64 steps in operand order, once per k-grid column; the field is applied to the accumulators.
 //
 // Current: J_a = sum_q sum_n coef(a, q, n) Z(q, n) with Z(q, n) = sum_k wp(k, q) x_n(k) over the real and
@@ -60,8 +60,10 @@ constexpr int kDfWarps = 8, kDfThreads = kDfWarps * 32;
 constexpr int kDfKS = 2;         // k-steps of the outer sums: box half-heights up to 3
 constexpr int kDfChunk = 64;     // steps per sums + propagation launch pair
 constexpr int kDfRing = 16;      // steps per flush of the current partials
+constexpr int kDfNj = 2;         // current axes
 constexpr int kDfMaxBox2 = 64;   // widest cell box along the second axis
 constexpr int kDfSumPts = 4;     // points per block of the sums kernel
+constexpr int kDfSumThreads = 192;
 
 __device__ __forceinline__ double2 df_mul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
@@ -136,19 +138,19 @@ struct DfData {
   const double* CW;  // [point][N2][nj][nt][16][4] (k-space solver: [N2]...)
 };
 
-// The sums of every column for the chunk's points: block = (kDfSumPts points, column).  A thread forms, for
-// one matrix and element pair (i, j), (j, i), the column sums G(n1) = sum_n2 p2(n2) X(n1, n2) of n1 = 0..3 at
-// the block's points (each table value loaded once for all of them) and writes the operands whole 32-byte
-// sectors at a time.
-__global__ void __launch_bounds__(192) dfrag_sums_kernel(SolveTables t, DfData d, int nt, double* GB, double* CW,
-                                                         int npts) {
-  __shared__ double2 q2[kDfSumPts][kDfMaxBox2];
-  __shared__ double2 w2[kDfSumPts][4];
-  const int sg = blockIdx.x / t.N2, m2 = blockIdx.x % t.N2, sl0 = sg * kDfSumPts;
-  const int ns = min(kDfSumPts, npts - sl0);
+// The sums of every column for the chunk's points: block = (kDfSumPts points, column).  A thread forms, for one
+// matrix, element pair (i, j), (j, i) and box row n1, the column sums G(n1) = sum_n2 p2(n2) X(n1, n2) at the
+// block's points.  It is bound by the latency of the table loads, so a thread keeps few accumulators and many
+// warps fit: with two rows and eight points per thread (168 registers) the chunk took 1.4 times as long.
+__global__ void __launch_bounds__(kDfSumThreads, 4) dfrag_sums_kernel(SolveTables t, DfData d, int nt, double* GB,
+                                                                      double* CW, int npts) {
+  constexpr int P = kDfSumPts;
+  __shared__ double2 q2[P][kDfMaxBox2];
+  __shared__ double2 w2[P][4];
+  const int m2 = blockIdx.x, sl0 = blockIdx.y * P, ns = min(P, npts - sl0);
   const int npw = 2 * t.np + 1, W1n = t.b1n, W2n = t.b2n, nw = t.nw, nw2 = t.nw2, half = (W1n - 1) / 2;
   const int nmat = 1 + t.nax, ne = nw * (nw + 1) / 2, ne4 = 4 * nt;
-  for (int idx = threadIdx.x; idx < kDfSumPts * (W2n + 4); idx += blockDim.x) {
+  for (int idx = threadIdx.x; idx < P * (W2n + 4); idx += blockDim.x) {
     const int j = idx / (W2n + 4), q = idx % (W2n + 4);
     const int s = (t.kmode ? 2 * t.step0 : t.step0) + sl0 + min(j, ns - 1);
     const double2* P2 = d.P + (size_t)s * 2 * npw + t.np + npw;
@@ -163,56 +165,50 @@ __global__ void __launch_bounds__(192) dfrag_sums_kernel(SolveTables t, DfData d
   __syncthreads();
   const double2 zero = make_double2(0.0, 0.0);
   const size_t gpt = (size_t)nmat * nt * kDfKS * 32, wpt = (size_t)t.nj * nt * 64;
-  for (int idx = threadIdx.x; idx < nmat * ne4; idx += blockDim.x) {
-    const int mat = idx / ne4, e = idx % ne4;
+  // Column j of packed element e (padding past ne: an empty element).
+  auto column = [&](int e) {
     int j = 0;
     while (df_elem(0, j + 1) <= e) ++j;
-    const int i = e - df_elem(0, j);
-    const bool on = e < ne, diag = i == j;
-    double re[kDfSumPts][8], im[kDfSumPts][8];
+    return j;
+  };
+  for (int idx = threadIdx.x; idx < 4 * nmat * ne4; idx += blockDim.x) {
+    // (neighbouring threads take the two rows n1 = q of a k-step: their 16-byte stores share a sector)
+    const int qs = idx & 1, e = (idx >> 1) % ne4, mk = (idx >> 1) / ne4, ks = mk & 1, mat = mk >> 1, q = 2 * ks + qs;
+    const int j = column(e), i = e - df_elem(0, j);
+    const bool on = e < ne && q <= half;
+    const double2* X = d.Xbox + (size_t)(mat * W1n + half + (on ? q : 0)) * W2n * nw2;
+    const int o0 = on ? i * nw + j : 0, o1 = on ? j * nw + i : 0;
+    double2 a[P], b[P];  // G(q) of (i, j) and of (j, i)
 #pragma unroll
-    for (int s = 0; s < kDfSumPts; ++s)
+    for (int s = 0; s < P; ++s) a[s] = b[s] = zero;
+    if (on) {
+      double2 x = X[o0], y = X[o1];
+#pragma unroll 1
+      for (int n = 0; n < W2n; ++n) {
+        // (the next cell's table values are on their way while this one's are used)
+        const int n1 = min(n + 1, W2n - 1) * nw2;
+        const double2 xn = X[n1 + o0], yn = X[n1 + o1];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) re[s][k] = im[s][k] = 0.0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      if (on && q <= half) {
-        const double2* X = d.Xbox + (size_t)(mat * W1n + half + q) * W2n * nw2;
-        double2 a[kDfSumPts], b[kDfSumPts];
-#pragma unroll
-        for (int s = 0; s < kDfSumPts; ++s) a[s] = b[s] = zero;
-        for (int n = 0; n < W2n; ++n) {
-          const double2 x = X[(size_t)n * nw2 + i * nw + j], y = X[(size_t)n * nw2 + j * nw + i];
-#pragma unroll
-          for (int s = 0; s < kDfSumPts; ++s) {
-            a[s] = df_fmac(q2[s][n], x, a[s]);
-            b[s] = df_fmac(q2[s][n], y, b[s]);
-          }
+        for (int s = 0; s < P; ++s) {
+          const double2 pf = q2[s][n];
+          a[s] = df_fmac(pf, x, a[s]);
+          b[s] = df_fmac(pf, y, b[s]);
         }
-#pragma unroll
-        for (int s = 0; s < kDfSumPts; ++s) {
-          if (q == 0) {
-            re[s][0] = a[s].x;
-            im[s][0] = diag ? 0.0 : a[s].y;
-          } else {
-            re[s][q] = a[s].x + b[s].x;
-            im[s][q] = a[s].y - b[s].y;
-            re[s][3 + q] = -(a[s].y + b[s].y);
-            im[s][3 + q] = a[s].x - b[s].x;
-          }
-        }
+        x = xn;
+        y = yn;
       }
-    const size_t o = ((size_t)mat * nt + e / 4) * kDfKS * 32 + 8 * (e % 4);
+    }
+    double* dst = GB + ((size_t)sl0 * t.N2 + m2) * gpt + (((size_t)mat * nt + e / 4) * kDfKS + ks) * 32 + 8 * (e % 4) + 2 * qs;
 #pragma unroll
-    for (int s = 0; s < kDfSumPts; ++s)
+    for (int s = 0; s < P; ++s)
       if (s < ns) {
-        double2* dst = reinterpret_cast<double2*>(GB + ((size_t)(sl0 + s) * t.N2 + m2) * gpt + o);
-#pragma unroll
-        for (int ks = 0; ks < 2; ++ks) {
-          dst[16 * ks + 0] = make_double2(re[s][4 * ks], re[s][4 * ks + 1]);
-          dst[16 * ks + 1] = make_double2(re[s][4 * ks + 2], re[s][4 * ks + 3]);
-          dst[16 * ks + 2] = make_double2(im[s][4 * ks], im[s][4 * ks + 1]);
-          dst[16 * ks + 3] = make_double2(im[s][4 * ks + 2], im[s][4 * ks + 3]);
+        double2* o = reinterpret_cast<double2*>(dst + (size_t)s * t.N2 * gpt);
+        if (q == 0) {
+          o[0] = make_double2(a[s].x, 0.0);
+          o[2] = make_double2(i == j ? 0.0 : a[s].y, 0.0);
+        } else {
+          o[0] = make_double2(a[s].x + b[s].x, -(a[s].y + b[s].y));
+          o[2] = make_double2(a[s].y - b[s].y, a[s].x - b[s].x);
         }
       }
   }
@@ -221,15 +217,17 @@ __global__ void __launch_bounds__(192) dfrag_sums_kernel(SolveTables t, DfData d
   const int nwp = t.kmode ? (sl0 == 0 ? 1 : 0) : ns;  // points whose window this block writes
   for (int idx = threadIdx.x; nwp > 0 && idx < t.nj * 4 * ne4; idx += blockDim.x) {
     const int e = idx % ne4, aq = idx / ne4;
-    int j = 0;
-    while (df_elem(0, j + 1) <= e) ++j;
-    const int i = e - df_elem(0, j);
+    const int j = column(e), i = e - df_elem(0, j);
+    // (the sums are linear in the tables: x and y of the window first)
     double2 x[4], y[4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
-      x[n] = e < ne ? d.Xwin[(size_t)(aq * 4 + n) * nw2 + i * nw + j] : zero;
-      y[n] = e < ne && i != j ? d.Xwin[(size_t)(aq * 4 + n) * nw2 + j * nw + i] : zero;
+      const double2 u = e < ne ? d.Xwin[(size_t)(aq * 4 + n) * nw2 + i * nw + j] : zero;
+      const double2 v = e < ne && i != j ? d.Xwin[(size_t)(aq * 4 + n) * nw2 + j * nw + i] : zero;
+      x[n] = make_double2(u.x + v.x, u.y + v.y);
+      y[n] = i == j ? zero : make_double2(u.y - v.y, v.x - u.x);
     }
+#pragma unroll 2
     for (int s = 0; s < nwp; ++s) {
       double2 a = zero, b = zero;
 #pragma unroll
@@ -239,20 +237,23 @@ __global__ void __launch_bounds__(192) dfrag_sums_kernel(SolveTables t, DfData d
       }
       const size_t blk = t.kmode ? (size_t)m2 : (size_t)(sl0 + s) * t.N2 + m2;
       double2* dst = reinterpret_cast<double2*>(CW + blk * wpt + (((size_t)(aq / 4) * nt + e / 4) * 16 + (aq % 4) * 4 + e % 4) * 4);
-      dst[0] = make_double2(a.x + b.x, a.y + b.y);
-      dst[1] = i == j ? zero : make_double2(a.y - b.y, b.x - a.x);
+      dst[0] = a;
+      dst[1] = b;
     }
   }
 }
+
+__host__ __device__ constexpr int df_current_warps(bool big, bool km) { return big || km ? 4 : 5; }
 
 // BIG: 9..12 orbitals (one k-point per warp, 8 per CTA); otherwise 3..8 (two per warp, 16 per CTA).
 template <bool BIG, int NAX, bool KM>
 struct DfShape {
   static constexpr int KPW = BIG ? 1 : 2, KPC = kDfWarps * KPW, MT = KPC / 8;
-  // Warps that form the current; the others form the next step's H.  The current is one product of
-  // KPC / 4 k-steps and NJ contractions per tile, H is (1 + NAX) products of 2 k-steps (two points per step
-  // in the k-space solver).
-  static constexpr int NCW = KM ? 2 : 3;
+  // Warps that form the current; the others form the next step's H.  A tile of the current (KPC / 4 products,
+  // four FP64 operations per axis and part) takes about twice a tile of H.  11 orbitals, 1024 steps of 150 x 150:
+  // 69.2 ms with 3, 66.0 with 4; 6 orbitals, 100 x 100: 54.1 with 3, 52.9 with 5, 54.8 with 6; 12 orbitals, k-space
+  // solver: 22.2 with 2, 20.8 with 4.
+  static constexpr int NCW = df_current_warps(BIG, KM);
 };
 
 template <bool BIG, int NAX, bool KM>
@@ -344,15 +345,15 @@ __global__ void __launch_bounds__(kDfThreads, 2)
 #pragma unroll
         for (int pb = 0; pb < NPT; ++pb) {
           if (KM && first && pb == 1) break;
-          double pa[MT][2];  // A[g][c]: a_c, b_{c+1} of k-point 8 m + g
+          double pa[MT][2];  // A[g][c] of the k-steps: part c % 2 of p(n1 = c / 2), p(n1 = 2 + c / 2) of k-point 8 m + g
 #pragma unroll
-          for (int m = 0; m < MT; ++m) {
-            const double2* tw = TW1 + (8 * m + g) * 4;
-            const double2 t0 = tw[c4], p0 = PQ[4 * pb + c4];
-            const double2 t1 = tw[(c4 + 1) & 3], p1 = PQ[4 * pb + ((c4 + 1) & 3)];
-            pa[m][0] = c4 <= half ? fma(t0.x, p0.x, -t0.y * p0.y) : 0.0;
-            pa[m][1] = c4 < half ? fma(t1.x, p1.y, t1.y * p1.x) : 0.0;
-          }
+          for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+              const int q = 2 * ks + (c4 >> 1);
+              const double2 tw = TW1[(8 * m + g) * 4 + q], pq = PQ[4 * pb + q];
+              pa[m][ks] = q > half ? 0.0 : (c4 & 1) ? fma(tw.x, pq.y, tw.y * pq.x) : fma(tw.x, pq.x, -tw.y * pq.y);
+            }
 #pragma unroll 2
           for (int n = wo; n < nt; n += nwo) {
             double acc[NMAT][MT][2];
@@ -396,15 +397,17 @@ __global__ void __launch_bounds__(kDfThreads, 2)
           }
         }
         double u[3] = {0.0, 0.0, 0.0}, s[3] = {0.0, 0.0, 0.0};
+        const double* rb = RHO + c4 * rhos + g;
+        const double* cw = CW + (h * 4 + c4) * 4;
 #pragma unroll 2
         for (int n = wc; n < nt; n += NCW) {
           double z[2] = {0.0, 0.0};
 #pragma unroll
-          for (int ks = 0; ks < KPC / 4; ++ks) dmma(z, wa[ks], RHO[(4 * ks + c4) * rhos + 8 * n + g]);
+          for (int ks = 0; ks < KPC / 4; ++ks) dmma(z, wa[ks], rb[4 * ks * rhos + 8 * n]);
 #pragma unroll
-          for (int a = 0; a < 3; ++a)
+          for (int a = 0; a < kDfNj; ++a)
             if (a < nj) {
-              const double2* cf = reinterpret_cast<const double2*>(CW + (((size_t)a * nt + n) * 16 + h * 4 + c4) * 4);
+              const double2* cf = reinterpret_cast<const double2*>(cw + (a * nt + n) * 64);
               const double2 cx = cf[0], cy = cf[1];
               u[a] = fma(cx.x, z[0], fma(cy.x, z[1], u[a]));
               s[a] = fma(cx.y, z[0], fma(cy.y, z[1], s[a]));
@@ -671,13 +674,13 @@ DfKernel df_kernel(const SolveTables& t) {
 }
 int df_kpc(const SolveTables& t) { return t.nw > 8 ? 8 : 16; }
 DfLayout df_layout(const SolveTables& t) {
-  return DfLayout(t.nw, t.nax, t.nj, df_kpc(t), t.kmode != 0, t.kmode ? 2 : 3);
+  return DfLayout(t.nw, t.nax, t.nj, df_kpc(t), t.kmode != 0, df_current_warps(t.nw > 8, t.kmode != 0));
 }
 
 }  // namespace
 
 // The solves this kernel takes: 3..12 orbitals, a Hermitian placement whose box is symmetric about zero, at
-// most 7 cells high (two k-steps) and 63 wide, and at least one field axis.  Over that whole range it is
+// most 7 cells high (two k-steps) and 63 wide, at least one field axis and at most two current axes.  Over that whole range it is
 // faster than the element-group kernel, which keeps the others: 512 steps of a 60 x 60 grid, two axes,
 // element groups / this kernel: 3 orbitals 4.7 / 2.5 ms, 4: 4.2 / 2.6, 5: 9.2 / 2.7, 6: 9.8 / 2.9, 8: 21.8 / 3.3,
 // 9: 27.3 / 7.1, 10: 34.4 / 7.4, 12: 28.8 / 8.2 (k-space solver 3: 7.8 / 2.7, 8: 38.4 / 3.7, 12: 36.2 / 11.1; 20 x 20,
@@ -685,7 +688,7 @@ DfLayout df_layout(const SolveTables& t) {
 bool plan_dfrag(const SolveTables& t, int sm_count, LaunchShape* out) {
   if (const char* env = std::getenv("HHG_DFRAG"))
     if (env[0] == '0') return false;
-  if (t.nw < 3 || t.nw > 12 || t.nax < 1 || !t.hermitian) return false;
+  if (t.nw < 3 || t.nw > 12 || t.nax < 1 || t.nj > kDfNj || !t.hermitian) return false;
   if (t.b1n > 7 || t.b1n % 2 == 0 || t.b1lo != -(t.b1n - 1) / 2) return false;
   if (t.b2n > 63 || t.b2n % 2 == 0 || t.b2lo != -(t.b2n - 1) / 2) return false;
   const DfLayout L = df_layout(t);
@@ -734,8 +737,7 @@ int launch_dfrag(const SolveTables& t, const GroupTables& gt, const LaunchShape&
     tc.step0 = c0;
     tc.step1 = std::min(c0 + s.pre_chunk, t.step1);
     const int npts = t.kmode ? 2 * (tc.step1 - c0) + 1 : tc.step1 - c0;
-    const int groups = (npts + kDfSumPts - 1) / kDfSumPts;
-    dfrag_sums_kernel<<<groups * t.N2, 192, 0, stream>>>(tc, d, L.nt, GB, CW, npts);
+    dfrag_sums_kernel<<<dim3(t.N2, (npts + kDfSumPts - 1) / kDfSumPts), kDfSumThreads, 0, stream>>>(tc, d, L.nt, GB, CW, npts);
     kern<<<s.ctas, s.threads, s.smem, stream>>>(tc, d, s.vctas, rho, Jpart);
     launches += 2;
   }
