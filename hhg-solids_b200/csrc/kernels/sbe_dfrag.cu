@@ -95,6 +95,11 @@ __device__ __forceinline__ void df_cp_wait() { asm volatile("cp.async.wait_all;"
 // Element (i <= j) of a Hermitian matrix: packed upper triangle by columns, the same for any orbital count.
 __host__ __device__ constexpr int df_elem(int i, int j) { return j * (j + 1) / 2 + i; }
 
+// Window coefficients read through L1 instead of staged: the k-space solver's are the same for all steps, and with
+// 9..12 orbitals and two axes staging them leaves one CTA on an SM at 12 orbitals (64 x 64, 1024 steps: 20.5 ms
+// staged, 17.0 not; 11 orbitals, where both fit twice, 8.0 and 8.1 for 512 steps).
+__host__ __device__ constexpr bool df_coef_global(bool big, int nax, bool km) { return km && big && nax >= 2; }
+
 // Shapes shared by the kernels and the planner (nt: 8-column tiles of the elements' parts).
 struct DfLayout {
   int nt, hks, rhos;   // double2 per k-point and sample of H; doubles per k-point of the staged state
@@ -113,7 +118,7 @@ struct DfLayout {
     GB = b;
     b += (km ? 2 : 1) * gpt * 8;
     CW = b;
-    b += wpt * 8;
+    if (!df_coef_global(nw > 8, nax, km)) b += wpt * 8;
     RHO = b;
     b += (size_t)kpc * rhos * 8;
     TW1 = b;
@@ -398,7 +403,8 @@ __global__ void __launch_bounds__(kDfThreads, 2)
         }
         double u[3] = {0.0, 0.0, 0.0}, s[3] = {0.0, 0.0, 0.0};
         const double* rb = RHO + c4 * rhos + g;
-        const double* cw = CW + (h * 4 + c4) * 4;
+        constexpr bool CG = df_coef_global(BIG, NAX, KM);
+        const double* cw = (CG ? d.CW + (size_t)m2 * L.wpt : CW) + (h * 4 + c4) * 4;
 #pragma unroll 2
         for (int n = wc; n < nt; n += NCW) {
           double z[2] = {0.0, 0.0};
@@ -408,7 +414,7 @@ __global__ void __launch_bounds__(kDfThreads, 2)
           for (int a = 0; a < kDfNj; ++a)
             if (a < nj) {
               const double2* cf = reinterpret_cast<const double2*>(cw + (a * nt + n) * 64);
-              const double2 cx = cf[0], cy = cf[1];
+              const double2 cx = CG ? __ldg(cf) : cf[0], cy = CG ? __ldg(cf + 1) : cf[1];
               u[a] = fma(cx.x, z[0], fma(cy.x, z[1], u[a]));
               s[a] = fma(cx.y, z[0], fma(cy.y, z[1], s[a]));
             }
@@ -449,7 +455,7 @@ __global__ void __launch_bounds__(kDfThreads, 2)
       __syncthreads();
       fetch_point(KM ? 2 * step0 : step0, 0);
       fetch_field(step0);
-      if (KM) fetch_window(step0);
+      if (KM && !df_coef_global(BIG, NAX, KM)) fetch_window(step0);
       // This warp's states.
       double2 rT[KPW][2], rU[KPW];
       double rV[KPW];
