@@ -32,6 +32,26 @@
 
 namespace mtile {
 
+// Two FP32 values in one 64-bit register pair, and d = a b + c on both (fma.rn.f32x2: each half rounds as fmaf).
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(F2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+  return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
 // Waits until at most one committed group of this thread's cp.async copies is still in flight.
 __device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
@@ -294,23 +314,34 @@ __global__ void __launch_bounds__(128, 3)
           }
           __syncwarp();
           // P = H X on the tile: P(i, j) = sum_l H(i, l) X(l, j), H(i, l) from row l of the transposed H.
+          // Each complex multiply-add is two packed ones, h.x (x, y) then h.y (-y, x): the roundings and their
+          // order of four scalar ones.
           float2 P[9];
+          {
+            F2 acc[9];
 #pragma unroll
-          for (int u = 0; u < 9; ++u) P[u] = fzero;
+            for (int u = 0; u < 9; ++u) acc[u] = pack2(0.f, 0.f);
 #pragma unroll
-          for (int l = 0; l < NW; ++l) {
-            const float2* hr = Hk + l * MS + i0;
-            const float2* xr = Xk + l * MS + j0;
-            const float2 h0 = hr[0], h1 = hr[1], h2 = hr[2], x0 = xr[0], x1 = xr[1], x2 = xr[2];
-            P[0] = fmac(h0, x0, P[0]);
-            P[1] = fmac(h0, x1, P[1]);
-            P[2] = fmac(h0, x2, P[2]);
-            P[3] = fmac(h1, x0, P[3]);
-            P[4] = fmac(h1, x1, P[4]);
-            P[5] = fmac(h1, x2, P[5]);
-            P[6] = fmac(h2, x0, P[6]);
-            P[7] = fmac(h2, x1, P[7]);
-            P[8] = fmac(h2, x2, P[8]);
+            for (int l = 0; l < NW; ++l) {
+              const float2* hr = Hk + l * MS + i0;
+              const float2* xr = Xk + l * MS + j0;
+              F2 xa[3], xb[3];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) {
+                const float2 q = xr[c];
+                xa[c] = pack2(q.x, q.y);
+                xb[c] = pack2(-q.y, q.x);
+              }
+#pragma unroll
+              for (int a = 0; a < 3; ++a) {
+                const float2 h = hr[a];
+                const F2 hx = pack2(h.x, h.x), hy = pack2(h.y, h.y);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) acc[3 * a + c] = fma2(hy, xb[c], fma2(hx, xa[c], acc[3 * a + c]));
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < 9; ++u) P[u] = unpack2(acc[u]);
           }
           __syncwarp();  // every lane of the k-point has read X
 #pragma unroll
