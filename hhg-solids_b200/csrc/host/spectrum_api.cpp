@@ -2,6 +2,7 @@
 // for a solve's recorded current or for caller-supplied currents.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -9,9 +10,38 @@
 #include "swe_sim.hpp"
 
 using hhg::check_cuda;
-using hhg::DevBuf;
 
 namespace {
+
+// Device workspace of one call, from the device's stream-ordered pool (as a solve's buffers), which is asked to
+// keep kKeepBytes between calls if it keeps less: a cudaMalloc and cudaFree per buffer and call took 1 to 30 ms a
+// call, both wait for the whole device, and the transform of a solve's current takes 0.05.  Allocated and freed in
+// the order of the call's stream, so calls of several threads and streams do not share memory that is in use.
+constexpr uint64_t kKeepBytes = uint64_t(256) << 20;
+
+void keep_pool_memory() {
+  int dev = 0;
+  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  cudaMemPool_t pool = nullptr;
+  check_cuda(cudaDeviceGetDefaultMemPool(&pool, dev), "cudaDeviceGetDefaultMemPool");
+  uint64_t keep = 0;
+  check_cuda(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolGetAttribute");
+  if (keep >= kKeepBytes) return;
+  keep = kKeepBytes;
+  check_cuda(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+}
+
+struct Workspace {
+  char* p = nullptr;
+  cudaStream_t stream;
+  Workspace(size_t bytes, cudaStream_t s) : stream(s) {
+    keep_pool_memory();
+    check_cuda(cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, s), "cudaMallocAsync");
+  }
+  ~Workspace() { cudaFreeAsync(p, stream); }
+  Workspace(const Workspace&) = delete;
+  Workspace& operator=(const Workspace&) = delete;
+};
 
 // S = fftshift(fft(ifftshift(gradient(J, h)))) for `count` host signals of length n.
 void spectrum_host(const double2* J, int n, int count, double h, double2* S, cudaStream_t stream) {
@@ -19,14 +49,13 @@ void spectrum_host(const double2* J, int n, int count, double h, double2* S, cud
   if (count < 1) throw std::runtime_error("spectrum: no signals");
   if (!(h > 0.0)) throw std::runtime_error("spectrum: the sample spacing must be positive");
   const size_t total = (size_t)n * count;
-  DevBuf<double2> dJ, dS, dT;
-  dJ.alloc(total);
-  dS.alloc(total);
-  dT.alloc(total);
-  check_cuda(cudaMemcpyAsync(dJ.p, J, sizeof(double2) * total, cudaMemcpyHostToDevice, stream), "H2D");
-  if (hhg::spectrum_device(dJ.p, n, count, h, dS.p, dT.p, stream) < 0)
+  Workspace ws(sizeof(double2) * (3 * total + n), stream);  // J, S, scratch and the table of roots
+  double2* dJ = reinterpret_cast<double2*>(ws.p);
+  double2 *dS = dJ + total, *dT = dS + total;
+  check_cuda(cudaMemcpyAsync(dJ, J, sizeof(double2) * total, cudaMemcpyHostToDevice, stream), "H2D");
+  if (hhg::spectrum_device(dJ, n, count, h, dS, dT, stream) < 0)
     throw std::runtime_error("spectrum: launch failed: " + std::string(cudaGetErrorString(cudaGetLastError())));
-  check_cuda(cudaMemcpyAsync(S, dS.p, sizeof(double2) * total, cudaMemcpyDeviceToHost, stream), "D2H");
+  check_cuda(cudaMemcpyAsync(S, dS, sizeof(double2) * total, cudaMemcpyDeviceToHost, stream), "D2H");
   check_cuda(cudaStreamSynchronize(stream), "spectrum");
 }
 
@@ -61,15 +90,25 @@ int HHG_harmonic_intensities(const hhg_cdouble* S, int n, int count, double tmax
     if (n < 2 || count < 1 || nh < 1) throw std::runtime_error("HHG_harmonic_intensities: empty input");
     if (!(tmax_fs > 0.0) || !(lambda_nm > 0.0))
       throw std::runtime_error("HHG_harmonic_intensities: tmax and lambda must be positive");
-    const size_t total = (size_t)n * count;
-    DevBuf<double2> dS;
-    DevBuf<double> dI;
-    dS.alloc(total);
-    dI.alloc((size_t)count * nh);
-    check_cuda(cudaMemcpy(dS.p, S, sizeof(double2) * total, cudaMemcpyHostToDevice), "H2D");
-    if (hhg::harmonics_device(dS.p, n, count, tmax_fs, lambda_nm, nh, dI.p, nullptr) != 0)
+    // Only the samples the windows can hold go to the device (a tenth of a 90 fs pulse's for 25 harmonics).
+    int i0 = 0, ni = 0;
+    hhg::harmonics_range(n, tmax_fs, lambda_nm, nh, &i0, &ni);
+    if (ni == 0) {
+      std::fill(I, I + (size_t)count * nh, 0.0);
+      return 0;
+    }
+    std::vector<double2> part((size_t)count * ni);
+    const double2* src = reinterpret_cast<const double2*>(S);
+    for (int b = 0; b < count; ++b) std::copy_n(src + (size_t)b * n + i0, ni, part.data() + (size_t)b * ni);
+    cudaStream_t stream = nullptr;
+    Workspace ws(sizeof(double2) * part.size() + sizeof(double) * (size_t)count * nh, stream);
+    double2* dS = reinterpret_cast<double2*>(ws.p);
+    double* dI = reinterpret_cast<double*>(dS + part.size());
+    check_cuda(cudaMemcpyAsync(dS, part.data(), sizeof(double2) * part.size(), cudaMemcpyHostToDevice, stream), "H2D");
+    if (hhg::harmonics_device(dS, n, i0, ni, count, tmax_fs, lambda_nm, nh, dI, stream) != 0)
       throw std::runtime_error("HHG_harmonic_intensities: launch failed");
-    check_cuda(cudaMemcpy(I, dI.p, sizeof(double) * (size_t)count * nh, cudaMemcpyDeviceToHost), "D2H");
+    check_cuda(cudaMemcpyAsync(I, dI, sizeof(double) * (size_t)count * nh, cudaMemcpyDeviceToHost, stream), "D2H");
+    check_cuda(cudaStreamSynchronize(stream), "HHG_harmonic_intensities");
     return 0;
   } catch (const std::exception& e) {
     hhg::set_thread_error(e.what());

@@ -6,10 +6,13 @@
 //
 // The FFT is a batched mixed-radix Stockham transform (autosorting, so no bit reversal): n is
 // factored into radices 4, 2, 3, 5 and any remaining prime, and each pass reads the previous pass's
-// buffer and writes the other.  For a pass of radix R after a product Ns of earlier radices, thread
+// buffer and writes the other.  For a pass of radix R after a product Ns of earlier radices, butterfly
 // j (of n/R) takes the R inputs j + r n/R, multiplies input r by e^{-2 pi i r (j mod Ns) / (Ns R)},
 // forms their length-R DFT and writes output q to (j div Ns) Ns R + (j mod Ns) + q Ns.  The first pass
 // reads the gradient of the current through the ifftshift, the last one writes through the fftshift.
+// A block runs all passes of one signal in shared memory (up to 7040 samples; longer ones go pass by pass
+// through global memory).  Radices up to 8 take a thread per butterfly, larger ones a thread per output, and all
+// factors come from one table of the n-th roots: a radix-4093 pass was one thread with a sincospi per term.
 #include <cuda_runtime.h>
 
 #include <cstdio>
@@ -19,6 +22,14 @@
 
 namespace hhg {
 namespace {
+
+// Samples [lo, hi) that can hold orders between a and b: two more on either side than the axis says.
+__host__ __device__ inline void harmonic_window(int n, double tmax, double w0, double a, double b, int* lo, int* hi) {
+  const double wmax = n * (2.0 * M_PI / tmax) / 2.0, step = n > 1 ? 2.0 * wmax / (double)(n - 1) : 1.0;
+  const double x = floor((a * w0 + wmax) / step) - 2.0, y = ceil((b * w0 + wmax) / step) + 3.0;
+  *lo = x < 0.0 ? 0 : (x > (double)n ? n : (int)x);
+  *hi = y < 0.0 ? 0 : (y > (double)n ? n : (int)y);
+}
 
 __device__ __forceinline__ double2 sp_mul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
@@ -46,64 +57,134 @@ __device__ __forceinline__ double2 sp_fma(double2 a, double2 w, double2 acc) {
   return make_double2(fma(a.x, w.x, fma(-a.y, w.y, acc.x)), fma(a.x, w.y, fma(a.y, w.x, acc.y)));
 }
 
-// One Stockham pass of radix R over `count` signals of length n.  first: read gradients of J
-// through the ifftshift; last: write through the fftshift.
-__global__ void stockham_pass_kernel(const double2* in, double2* out, const double2* J, int n, int count, int R,
-                                     int Ns, int first, int last, double h) {
-  const long long total = (long long)count * (n / R);
-  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= total) return;
-  const int b = (int)(gid / (n / R)), j = (int)(gid % (n / R));
-  const double2* src = first ? nullptr : in + (size_t)b * n;
-  const double2* Jb = J + (size_t)b * n;
-  double2* dst = out + (size_t)b * n;
-  const int k = j % Ns, stride = n / R;
-  const int base = (j / Ns) * Ns * R + k;
-  const long long span = (long long)Ns * R;
-  auto input = [&](int r) {
-    const double2 x = first ? sp_grad_shifted(Jb, n, j + r * stride, h) : src[j + r * stride];
-    return r == 0 ? x : sp_mul(x, sp_twiddle((long long)r * k % span, span));
-  };
-  auto store = [&](int q, double2 acc) {
-    const int o = base + q * Ns;
-    dst[last ? (o + n / 2) % n : o] = acc;  // fftshift: element i of the result is X[(i - n/2) mod n]
-  };
+// w[k] = e^{-2 pi i k / n}.
+__global__ void roots_kernel(double2* w, int n) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) w[k] = sp_twiddle(k, n);
+}
+
+// Work item `it` of a pass: a butterfly (radix up to 8: n / R items) or one output of one (n items).
+// in(i): input i of the pass; out(o, value).  All factors are powers of the n-th root w.
+template <typename In, typename Out>
+__device__ __forceinline__ void stockham_item(int it, int n, int R, int Ns, const double2* w, In&& in, Out&& out) {
   constexpr int kMaxReg = 8;
+  const int stride = n / R;
+  const int j = R <= kMaxReg ? it : it % stride, k = j % Ns, base = (j / Ns) * Ns * R + k;
+  const int tk = k * (n / (Ns * R));  // input r's factor: root r tk (r k < Ns R, so r tk < n)
+  const int fq = stride;              // the DFT's root: e^{-2 pi i / R} = w^(n / R)
   if (R <= kMaxReg) {
     double2 v[kMaxReg];
-    for (int r = 0; r < R; ++r) v[r] = input(r);
-    for (int q = 0; q < R; ++q) {
-      double2 acc = v[0];
-      for (int r = 1; r < R; ++r) acc = sp_fma(v[r], sp_twiddle((long long)r * q % R, R), acc);
-      store(q, acc);
-    }
+#pragma unroll
+    for (int r = 0; r < kMaxReg; ++r)
+      if (r < R) {
+        v[r] = in(j + r * stride);
+        if (r > 0) v[r] = sp_mul(v[r], w[r * tk]);
+      }
+#pragma unroll
+    for (int q = 0; q < kMaxReg; ++q)
+      if (q < R) {
+        double2 acc = v[0];
+#pragma unroll
+        for (int r = 1; r < kMaxReg; ++r)
+          if (r < R) acc = sp_fma(v[r], w[r * q % R * fq], acc);
+        out(base + q * Ns, acc);
+      }
   } else {
-    // Large prime radix: direct DFT, inputs re-read for every output.
-    for (int q = 0; q < R; ++q) {
-      double2 acc = make_double2(0.0, 0.0);
-      for (int r = 0; r < R; ++r) acc = sp_fma(input(r), sp_twiddle((long long)r * q % R, R), acc);
-      store(q, acc);
+    const int q = it / stride;
+    double2 acc = make_double2(0.0, 0.0);
+    int rq = 0, rt = 0;  // r q mod R, r tk mod n
+    for (int r = 0; r < R; ++r) {
+      const double2 x = in(j + r * stride);
+      acc = sp_fma(r == 0 ? x : sp_mul(x, w[rt]), w[rq * fq], acc);
+      rq += q;
+      if (rq >= R) rq -= R;
+      rt += tk;
     }
+    out(base + q * Ns, acc);
   }
 }
 
-// I[b][h'] for odd harmonics h = 2 h' + 1: sum of |S|^2 over order in (h - 1/2, h + 1/2).
-__global__ void harmonics_kernel(const double2* S, int n, int count, double tmax, double w0, int nh, double* I) {
-  const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+// Radices of a length (a length below 2^31 has at most 30 factors).
+struct Radices {
+  int count, r[30];
+};
+constexpr int kBlockSamples = 7040;  // two buffers of a signal in 220 KB of shared memory
+constexpr int kBlockThreads = 512;
+
+// A block per signal, all passes in shared memory.
+__global__ void __launch_bounds__(kBlockThreads) stockham_block_kernel(const double2* J, double2* S, const double2* w,
+                                                                       int n, Radices rad, double h) {
+  extern __shared__ __align__(16) double2 sp_buf[];
+  const double2* Jb = J + (size_t)blockIdx.x * n;
+  double2* Sb = S + (size_t)blockIdx.x * n;
+  int Ns = 1;
+  for (int p = 0; p < rad.count; ++p) {
+    const int R = rad.r[p], items = R <= 8 ? n / R : n;
+    const bool first = p == 0, last = p == rad.count - 1;
+    const double2* src = sp_buf + (size_t)(p & 1) * n;
+    double2* dst = sp_buf + (size_t)(~p & 1) * n;
+    // (a large first radix reads each input for every output: the gradient is formed once)
+    if (first && R > 8) {
+      for (int i = threadIdx.x; i < n; i += kBlockThreads) sp_buf[i] = sp_grad_shifted(Jb, n, i, h);
+      __syncthreads();
+    }
+    for (int it = threadIdx.x; it < items; it += kBlockThreads)
+      stockham_item(
+          it, n, R, Ns, w, [&](int i) { return first && R <= 8 ? sp_grad_shifted(Jb, n, i, h) : src[i]; },
+          [&](int o, double2 v) {
+            if (last)
+              Sb[o + n / 2 < n ? o + n / 2 : o + n / 2 - n] = v;  // fftshift: element i of the result is X[(i - n/2) mod n]
+            else
+              dst[o] = v;
+          });
+    Ns *= R;
+    __syncthreads();
+  }
+}
+
+// One pass over `count` signals through global memory.  first: read gradients of J through the ifftshift; last:
+// write through the fftshift.
+__global__ void stockham_pass_kernel(const double2* in, double2* out, const double2* J, const double2* w, int n, int count,
+                                     int R, int Ns, int first, int last, double h) {
+  const int items = R <= 8 ? n / R : n;
+  const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= (long long)count * items) return;
+  const int b = (int)(gid / items), it = (int)(gid % items);
+  const double2* src = first ? nullptr : in + (size_t)b * n;
+  const double2* Jb = J + (size_t)b * n;
+  double2* dst = out + (size_t)b * n;
+  stockham_item(
+      it, n, R, Ns, w, [&](int i) { return first ? sp_grad_shifted(Jb, n, i, h) : src[i]; },
+      [&](int o, double2 v) { dst[last ? (o + n / 2) % n : o] = v; });
+}
+
+// I[b][h'] for odd harmonics h = 2 h' + 1: sum of |S|^2 over order in (h - 1/2, h + 1/2).  A warp per value; the
+// samples of the window are found from the order axis (with a margin for its rounding) and each is tested as
+// written above.  S holds the samples i0 .. i0 + ni - 1 of each signal.  (A thread per value that tested all n
+// samples took 1 ms for any number of signals.)
+__global__ void harmonics_kernel(const double2* S, int n, int i0, int ni, int count, double tmax, double w0, int nh,
+                                 double* I) {
+  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (gid >= count * nh) return;
   const int b = gid / nh, hh = gid % nh;
   const double h = 2.0 * hh + 1.0;
   const double wmax = n * (2.0 * M_PI / tmax) / 2.0;
   const double step = n > 1 ? 2.0 * wmax / (double)(n - 1) : 0.0;
+  int lo, hi;
+  harmonic_window(n, tmax, w0, h - 0.5, h + 0.5, &lo, &hi);
+  lo = max(lo, i0);
+  hi = min(hi, i0 + ni);
   double acc = 0.0;
-  for (int i = 0; i < n; ++i) {
+  for (int i = lo + lane; i < hi; i += 32) {
     const double order = (-wmax + step * i) / w0;
     if (order > h - 0.5 && order < h + 0.5) {
-      const double2 s = S[(size_t)b * n + i];
+      const double2 s = S[(size_t)b * ni + (i - i0)];
       acc += s.x * s.x + s.y * s.y;
     }
   }
-  I[gid] = acc;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (lane == 0) I[gid] = acc;
 }
 
 std::vector<int> factor_radices(int n) {
@@ -129,21 +210,33 @@ std::vector<int> factor_radices(int n) {
 
 }  // namespace
 
+// scratch: count n values and, after them, n for the table of roots.
 int spectrum_device(const double2* J, int n, int count, double h, double2* S, double2* scratch, cudaStream_t stream) {
   if (n < 2 || count < 1 || h <= 0.0) return -1;
   const std::vector<int> rad = factor_radices(n);
-  // Ping-pong between S and scratch so that the last pass lands in S.
   const int passes = (int)rad.size();
+  double2* w = scratch + (size_t)count * n;
+  roots_kernel<<<(n + 255) / 256, 256, 0, stream>>>(w, n);
+  if (n <= kBlockSamples) {
+    Radices r{};
+    r.count = passes;
+    for (int p = 0; p < passes; ++p) r.r[p] = rad[p];
+    const size_t smem = 2 * (size_t)n * sizeof(double2);
+    cudaFuncSetAttribute(stockham_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    stockham_block_kernel<<<count, kBlockThreads, smem, stream>>>(J, S, w, n, r, h);
+    return cudaGetLastError() == cudaSuccess ? passes : -1;
+  }
+  // Ping-pong between S and scratch so that the last pass lands in S.
   double2* bufs[2] = {S, scratch};
   int cur = passes % 2 == 1 ? 0 : 1;  // buffer written by the first pass
   int Ns = 1;
   const double2* prev = nullptr;
   for (int p = 0; p < passes; ++p) {
     const int R = rad[p];
-    const long long threads = (long long)count * (n / R);
+    const long long threads = (long long)count * (R <= 8 ? n / R : n);
     const int block = 128;
     const int grid = (int)((threads + block - 1) / block);
-    stockham_pass_kernel<<<grid, block, 0, stream>>>(prev, bufs[cur], J, n, count, R, Ns, p == 0, p == passes - 1, h);
+    stockham_pass_kernel<<<grid, block, 0, stream>>>(prev, bufs[cur], J, w, n, count, R, Ns, p == 0, p == passes - 1, h);
     prev = bufs[cur];
     cur ^= 1;
     Ns *= R;
@@ -151,12 +244,19 @@ int spectrum_device(const double2* J, int n, int count, double h, double2* S, do
   return cudaGetLastError() == cudaSuccess ? passes : -1;
 }
 
-int harmonics_device(const double2* S, int n, int count, double tmax, double lambda_nm, int nh, double* I,
+void harmonics_range(int n, double tmax, double lambda_nm, int nh, int* i0, int* ni) {
+  int lo, hi;
+  harmonic_window(n, tmax, 2.0 * M_PI * 300.0 / lambda_nm, 0.5, 2.0 * nh - 0.5, &lo, &hi);
+  *i0 = lo;
+  *ni = hi > lo ? hi - lo : 0;
+}
+
+int harmonics_device(const double2* S, int n, int i0, int ni, int count, double tmax, double lambda_nm, int nh, double* I,
                      cudaStream_t stream) {
   if (n < 2 || count < 1 || nh < 1 || tmax <= 0.0 || lambda_nm <= 0.0) return -1;
   const double w0 = 2.0 * M_PI * 300.0 / lambda_nm;
-  const int total = count * nh;
-  harmonics_kernel<<<(total + 127) / 128, 128, 0, stream>>>(S, n, count, tmax, w0, nh, I);
+  const long long warps = (long long)count * nh;
+  harmonics_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, stream>>>(S, n, i0, ni, count, tmax, w0, nh, I);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
