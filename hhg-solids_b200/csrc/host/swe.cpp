@@ -707,9 +707,9 @@ size_t SWESim::footprint_estimate() const {
   return b;
 }
 
-// The pinned [3][nt] host copy of the current, allocated at the first run rather than at setup: a
-// solve set up by a server while others run never needs it (page-locking allocations can wait for
-// the device).
+// The pinned [3][nt] host copy of the current, allocated at a setup's second run: a solve set up by a
+// server while others run, or run once, never needs it (page-locking allocations can wait for the
+// device).
 double2* SWESim::host_J() {
   if (!h_J || h_J_cap < (size_t)3 * nt) {
     if (h_J) cudaFreeHost(h_J);
@@ -748,11 +748,16 @@ void SWESim::run() {
   hhg::TraceRange range("hhg SWESim_run_simulation");
   if (!ready) throw std::runtime_error("SWESim_run_simulation: SWESim_init has not succeeded");
   check_cuda(cudaSetDevice(device), "cudaSetDevice");
-  double2* hJ = host_J();
+  // A setup's first run copies its current to pageable memory if no earlier setup left a pinned buffer:
+  // page-locking one takes 1 to 3 ms.
+  const bool first = first_run_gen != generation, unpinned = first && h_J_cap < (size_t)3 * nt;
+  std::vector<double2> pageable(unpinned ? 3 * (size_t)nt : 0);
+  double2* hJ = unpinned ? pageable.data() : host_J();
   // The time loop (src/swe.cpp:183-223) as one launch sequence: clear the current partials, the
   // propagation launches (a pair per chunk of steps for precomputed-sum shapes), the reduction and the
-  // copy of J to pinned host memory.  It is captured into a CUDA graph at the first run of a setup and
-  // replayed afterwards, so a run costs one graph launch.
+  // copy of J to the host.  A setup's first run launches it directly (a scan sets each angle up, runs it
+  // once and drops it: capturing and instantiating the 18 launches of a 40 x 40 solve took about 1 ms); the second
+  // captures it into a CUDA graph, which it and later ones replay, so that a run costs one graph launch.
   auto enqueue = [&] {
     // (external event records: inside a captured graph they record when the graph runs)
     check_cuda(cudaMemsetAsync(d_Jpart.p, 0, sizeof(double2) * d_Jpart.n, stream), "memset");
@@ -763,7 +768,7 @@ void SWESim::run() {
     check_cuda(cudaMemcpyAsync(hJ, d_J.p, sizeof(double2) * 3 * (size_t)nt, cudaMemcpyDeviceToHost, stream), "D2H");
     return n;
   };
-  if (!run_graphs_enabled()) {
+  if (!run_graphs_enabled() || first) {
     drop_run_graph();
     last_launches = enqueue();
   } else {
@@ -793,6 +798,7 @@ void SWESim::run() {
   check_cuda(cudaStreamSynchronize(stream), "run_simulation");
   check_cuda(cudaEventElapsedTime(&last_ms, ev0, ev1), "event time");
   check_cuda(cudaEventElapsedTime(&last_prop_ms, ev0, evm), "event time");
+  first_run_gen = generation;
   // The reference appends one sample per step to each Observable (src/observable.cpp:29);
   // SWESim_get_current returns the first nt of them.
   for (int a = 0; a < 3; ++a)
