@@ -764,13 +764,13 @@ constexpr int kPreChunk = 64;   // steps per precompute + propagate launch pair
 // Inner Wannier sums of every column for the steps [t.step0, t.step1): block (point group, m2) forms,
 // for kSumPts consecutive points s of the chunk, the box rows G_e = sum_q p2(q) X(mat, q1s + qq, q)_e
 // and the window rows, with the operations (and their order) of group_vctas's inner_sums, into
-// [s - t.step0][m2][row][nw2]; each thread loads a row's X values once for all of the block's points.
+// [s - t.step0][m2][row][nw][gr] (gr: the stride between an element's rows, nw or wider); each thread loads a row's X values once for all of the block's points.
 // For the k-space solver the points are 2 step0 ... 2 step1 and the window rows, the same for every
 // point, are written once per column ([m2][row][nw2], by the block of the first point).
 constexpr int kSumPts = 8;
 template <typename Real>
 __global__ void __launch_bounds__(256) group_sums_kernel(SolveTables t, GroupData<Real> d, int q1s, int nq1,
-                                                         int nbrows, int nwrows, typename Cx<Real>::T* Gpre,
+                                                         int nbrows, int nwrows, int gr, typename Cx<Real>::T* Gpre,
                                                          double2* GWpre, int npts) {
   using V = typename Cx<Real>::T;
   __shared__ V q2[kSumPts][kMaxPreBox];
@@ -804,9 +804,11 @@ __global__ void __launch_bounds__(256) group_sums_kernel(SolveTables t, GroupDat
       for (int j = 0; j < kSumPts; ++j)
         if (j < ns) acc[j] = fmac(q2[j][q], x, acc[j]);
     }
+    const size_t blk = (size_t)nbrows * t.nw * gr;
+    V* out = Gpre + ((size_t)sl0 * t.N2 + m2) * blk + (gr == t.nw ? idx : row * t.nw * gr + e / t.nw * gr + e % t.nw);
 #pragma unroll
     for (int j = 0; j < kSumPts; ++j)
-      if (j < ns) Gpre[((size_t)(sl0 + j) * t.N2 + m2) * nbrows * nw2 + idx] = acc[j];
+      if (j < ns) out[j * blk * t.N2] = acc[j];
   }
   const int nwp = t.kmode ? (sl0 == 0 ? 1 : 0) : ns;  // points whose window rows this block writes
   for (int idx = threadIdx.x; idx < nwrows * nw2; idx += blockDim.x) {
@@ -827,9 +829,9 @@ __global__ void __launch_bounds__(256) group_sums_kernel(SolveTables t, GroupDat
 // Launches group_sums_kernel over the npts points of the chunk that starts at t.step0.
 template <typename Real>
 void launch_group_sums(const SolveTables& t, const GroupData<Real>& d, int q1s, int nq1, int nbrows, int nwrows,
-                       typename Cx<Real>::T* Gpre, double2* GWpre, int npts, cudaStream_t stream) {
+                       int gr, typename Cx<Real>::T* Gpre, double2* GWpre, int npts, cudaStream_t stream) {
   const int groups = (npts + kSumPts - 1) / kSumPts;
-  group_sums_kernel<Real><<<groups * t.N2, 256, 0, stream>>>(t, d, q1s, nq1, nbrows, nwrows, Gpre, GWpre, npts);
+  group_sums_kernel<Real><<<groups * t.N2, 256, 0, stream>>>(t, d, q1s, nq1, nbrows, nwrows, gr, Gpre, GWpre, npts);
 }
 
 template <typename Real>
@@ -978,7 +980,7 @@ int launch_group_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
       tc.step0 = c0;
       tc.step1 = std::min(c0 + s.pre_chunk, t.step1);
       const int npts = KM ? 2 * (tc.step1 - c0) + 1 : tc.step1 - c0;
-      launch_group_sums<Real>(tc, d, gg.q1s, gg.nq1, gg.nbrows, gg.nwrows, Gpre, GWpre, npts, stream);
+      launch_group_sums<Real>(tc, d, gg.q1s, gg.nq1, gg.nbrows, gg.nwrows, t.nw, Gpre, GWpre, npts, stream);
       kern<<<s.ctas, s.threads, s.smem, stream>>>(tc, d, s.k_per_cta, s.group, s.box_sm, s.win_sm, s.vctas, rho, Jpart);
       launches += 2;
     }
@@ -1057,7 +1059,7 @@ int launch_frag_t(const SolveTables& t, const GroupTables& gt, const LaunchShape
     SolveTables tc = t;
     tc.step0 = c0;
     tc.step1 = std::min(c0 + s.pre_chunk, t.step1);
-    launch_group_sums<float>(tc, d, 3, 4, FG::NBROWS, FG::NWROWS, Gpre, GWpre, tc.step1 - c0, stream);
+    launch_group_sums<float>(tc, d, 3, 4, FG::NBROWS, FG::NWROWS, NW, Gpre, GWpre, tc.step1 - c0, stream);
     kern<<<s.ctas, s.threads, s.smem, stream>>>(tc, d, s.vctas, rho, Jpart);
     launches += 2;
   }
@@ -1092,7 +1094,7 @@ bool plan_mtile_t(const SolveTables& t, int sm_count, LaunchShape* out, char* wh
   out->box_sm = out->win_sm = 0;
   out->smem = FG::BYTES;
   out->pre_chunk = std::min(kPreChunk, t.nt);
-  const size_t gbytes = (size_t)FG::NBROWS * FG::NW2 * sizeof(float2), wbytes = (size_t)FG::NWROWS * FG::NW2 * sizeof(double2);
+  const size_t gbytes = (size_t)FG::NBROWS * FG::GE * sizeof(float2), wbytes = (size_t)FG::NWROWS * FG::NW2 * sizeof(double2);
   out->pre_bytes = KM ? (size_t)(2 * out->pre_chunk + 1) * t.N2 * gbytes + (size_t)t.N2 * wbytes
                       : (size_t)out->pre_chunk * t.N2 * (gbytes + wbytes);
   return true;
@@ -1105,7 +1107,7 @@ int launch_mtile_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
   if (!gt.pre || s.pre_chunk <= 0)
     throw std::runtime_error("tile kernel launch: needs its precomputed-sum scratch (GroupTables::pre)");
   GroupData<float> d = {gt.Xbox32, gt.P32, gt.T1_32, gt.T2_32, gt.Xwin64, gt.P64, gt.T1_64, gt.T2_64, nullptr, nullptr};
-  const size_t gbuf = (size_t)FG::NBROWS * FG::NW2;
+  const size_t gbuf = (size_t)FG::NBROWS * FG::GE;
   float2* Gpre = static_cast<float2*>(gt.pre);
   const size_t npts_max = KM ? 2 * (size_t)s.pre_chunk + 1 : (size_t)s.pre_chunk;
   double2* GWpre = reinterpret_cast<double2*>(Gpre + npts_max * t.N2 * gbuf);
@@ -1119,7 +1121,7 @@ int launch_mtile_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
     tc.step0 = c0;
     tc.step1 = std::min(c0 + s.pre_chunk, t.step1);
     const int npts = KM ? 2 * (tc.step1 - c0) + 1 : tc.step1 - c0;
-    launch_group_sums<float>(tc, d, 3, 4, FG::NBROWS, FG::NWROWS, Gpre, GWpre, npts, stream);
+    launch_group_sums<float>(tc, d, 3, 4, FG::NBROWS, FG::NWROWS, FG::GR, Gpre, GWpre, npts, stream);
     kern<<<s.ctas, s.threads, s.smem, stream>>>(tc, d, s.vctas, rho, Jpart);
     launches += 2;
   }
