@@ -40,10 +40,11 @@
 // A step has two phases between CTA barriers: the RK4 stages (each warp its own k-points), and the
 // current of the step (NCW warps) beside the H of the next one (the others).
 //
-// Measured on B200 (1965 MHz): 11 orbitals, 150 x 150, one field axis, 4096 steps 276 ms (a 16 x 16 frame with
+// Measured on B200 (1965 MHz): 11 orbitals, 150 x 150, one field axis, 4096 steps 262 ms (a 16 x 16 frame with
 // one k-point per warp at 208 registers, 8 warps per SM: 525 ms); 6 orbitals, 100 x 100, two axes, 4096 steps
-// 54 ms (element-group kernel 162 ms); 12 orbitals, 64 x 64, two axes, k-space solver, 1024 steps 22.3 ms
-// (element groups 72.6); 5 orbitals, 46 x 38, 1024 steps 3.8 ms (element groups 9.5).
+// 52.2 ms (element-group kernel 162 ms); 12 orbitals, 64 x 64, two axes, k-space solver, 1024 steps 17.1 ms
+// (element groups 72.6); 5 orbitals, 46 x 38, 1024 steps 3.7 ms (element groups 9.5).  The shared FP64/tensor
+// pipe is 81-83 % busy.
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>

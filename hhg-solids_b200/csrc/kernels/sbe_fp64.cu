@@ -16,7 +16,8 @@
 //
 // propagate_kpt_kernel<NW>  (nw <= 2, Hermitian placement): one thread per k-point, the whole
 //   state in registers; per-cell phases e^{-ik.R_c} (per thread, fixed) x e^{iA.R_c} (per step).
-// propagate_group_kernel    (any nw <= 16, FP64 or mixed precision): in sbe_group.cu.
+// Two orbitals on all but the smallest grids: sbe_kcol.cu (one orbital, larger boxes: sbe_kcol_any.cu); 3 to 12 orbitals
+// in FP64: sbe_dfrag.cu; the mixed form and everything else (any nw <= 16): sbe_group.cu.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
