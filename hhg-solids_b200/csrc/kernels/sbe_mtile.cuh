@@ -19,7 +19,8 @@
 //  * the lane forms its tile of P = H X in FP32 from rows l of both arrays (three H and three X
 //    values per l: 36 FMA per 6 loads, every load a broadcast to the lanes of its tile row or
 //    column);
-//  * P replaces X in shared memory, and k = -i (P - P^+) takes P^+ from the transposed tile;
+//  * k = -i (P - P^+) takes P^+ from the lane of the transposed tile, by shuffles or (Geom::SHFL) through the
+//    place of X in shared memory;
 //  * the RK4 sum and the next stage's X are formed in FP64 (X stored as FP32).
 // Only the k-point's lanes (within one warp) exchange data, so the stages need __syncwarp only; the CTA meets twice
 // per step for the current (its FP64 window rows copied in during the step, then the FP64 state staged
@@ -90,6 +91,10 @@ struct Geom {
   static constexpr bool SINGLE = !SHARE || NW2 > 4 * PL;
   static constexpr int NOUT = SINGLE ? 9 : 8;  // elements of H that a lane forms
   static constexpr int HMS = SINGLE ? MS : NWP + 1, HKS = SINGLE ? KS : NWP * HMS + 1;  // strides of H
+  // P^+ by shuffles between the lanes of transposed tiles, which saves half the exchange's wavefronts and two of four
+  // warp barriers per stage: 6 orbitals 9.51 -> 9.06 ms (150 x 150, 512 steps), k-space solver 2.87 -> 2.68, 11 orbitals
+  // 1 %.  12 orbitals keep it in shared memory (from 1 % faster to 2 % slower with shuffles).
+  static constexpr bool SHFL = NW < 12;
   static constexpr bool STAGED = NWP == 12;    // row factors formed once per CTA and point
   // Row stride and size of an inner-sum matrix: rows of 12 keep the tiles of a half warp in different banks, also
   // transposed (with rows of 11 three pairs of the 16 collide).
@@ -142,6 +147,7 @@ __global__ void __launch_bounds__(128, 3)
   const int step0 = t.step0, step1 = t.step1, npw = 2 * t.np + 1;
   const double dt = t.dt, prefac = 0.1666666666666 * dt;
   constexpr size_t gbuf = (size_t)FG::NBROWS * FG::GE, wbuf = (size_t)FG::NWROWS * NW2;
+  const int lt = lane - sub + sub % FG::TD * FG::TD + sub / FG::TD;  // the lane of the transposed tile
   float2* Hk = HS + kp * HKS;
   float2* Xk = XPb + kp * KS;
   const float2 fzero = make_float2(0.f, 0.f);
@@ -455,16 +461,20 @@ __global__ void __launch_bounds__(128, 3)
 #pragma unroll
             for (int u = 0; u < 9; ++u) P[u] = unpack2(acc[u]);
           }
-          __syncwarp();  // every lane of the k-point has read X
+          __syncwarp();  // every lane of the k-point has read X and H
+          if constexpr (!FG::SHFL) {
 #pragma unroll
-          for (int u = 0; u < 9; ++u) Xk[own(u)] = P[u];
-          __syncwarp();
+            for (int u = 0; u < 9; ++u) Xk[own(u)] = P[u];
+            __syncwarp();
+          }
           const double wgt = (st == 0 || st == 3) ? 1.0 : 2.0;
           const double cn = (st == 2 ? 1.0 : 0.5) * dt;
           float2 xn[9];
 #pragma unroll
           for (int u = 0; u < 9; ++u) {
-            const float2 pt = Xk[tra(u)];
+            const int ut = 3 * (u % 3) + u / 3;  // P(j, i): this place of the transposed tile
+            const float2 pt = FG::SHFL ? make_float2(__shfl_sync(0xffffffffu, P[ut].x, lt), __shfl_sync(0xffffffffu, P[ut].y, lt))
+                                       : Xk[tra(u)];
             const float kx = P[u].y + pt.y, ky = -(P[u].x - pt.x);  // k = -i (P - P^+)
             if (st == 0) {
               S[u] = make_double2((double)kx, (double)ky);
@@ -474,7 +484,7 @@ __global__ void __launch_bounds__(128, 3)
             }
             xn[u] = make_float2((float)(r[u].x + cn * (double)kx), (float)(r[u].y + cn * (double)ky));
           }
-          __syncwarp();  // every lane of the k-point has read P
+          if constexpr (!FG::SHFL) __syncwarp();  // every lane of the k-point has read P
           if (st < 3) {
 #pragma unroll
             for (int u = 0; u < 9; ++u) Xk[own(u)] = xn[u];
