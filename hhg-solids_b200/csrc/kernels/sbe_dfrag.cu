@@ -52,6 +52,7 @@
 
 #include "dmma.cuh"
 #include "sbe_device.h"
+#include "smem_limit.h"
 #include "warp_reduce.cuh"
 
 namespace hhg {
@@ -700,10 +701,7 @@ bool plan_dfrag(const SolveTables& t, int sm_count, LaunchShape* out) {
   if (t.b2n > 63 || t.b2n % 2 == 0 || t.b2lo != -(t.b2n - 1) / 2) return false;
   const DfLayout L = df_layout(t);
   DfKernel kern = df_kernel(t);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.bytes) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  if (!allow_shared_memory(kern, L.bytes)) return false;
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kDfThreads, L.bytes);
   if (occ < 1) return false;
@@ -737,7 +735,7 @@ int launch_dfrag(const SolveTables& t, const GroupTables& gt, const LaunchShape&
   double* CW = GB + pts_max * t.N2 * L.gpt;
   const DfData d = {gt.Xbox64, gt.Xwin64, gt.P64, gt.T1_64, gt.T2_64, GB, CW};
   DfKernel kern = df_kernel(t);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  allow_shared_memory(kern, s.smem);
   int launches = 0;
   for (int c0 = t.step0; c0 < t.step1; c0 += s.pre_chunk) {
     SolveTables tc = t;

@@ -24,6 +24,7 @@
 
 #include "sbe_device.h"
 #include "sbe_herm2.cuh"
+#include "smem_limit.h"
 
 namespace hhg {
 namespace {
@@ -484,7 +485,7 @@ bool plan_kpt(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem_
   threads = threads < 64 ? 64 : (threads > kKptMaxThreads ? kKptMaxThreads : threads);
   while (threads > 64 && kpt_smem(t, threads) > smem_max) threads -= 32;
   if (kpt_smem(t, threads) > smem_max) return false;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kpt_smem(t, threads));
+  allow_shared_memory(kern, kpt_smem(t, threads));
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, kpt_smem(t, threads));
   if (occ < 1) return false;
@@ -553,7 +554,7 @@ int launch_propagate_steps(const SolveTables& t, const GroupTables& gt, const La
   if (t.step0 >= t.step1) return 0;
   if (s.kernel == 0) {
     KptKernel kern = kpt_kernel_for(t);
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    allow_shared_memory(kern, s.smem);
     kern<<<s.ctas, s.threads, s.smem, stream>>>(t, s.vctas, rho, Jpart);
     return 1;
   }
@@ -587,7 +588,7 @@ void launch_reduce_current(const double2* Jpart, int vctas, int nt, int Nk, doub
 
 int launch_rho0_fp64(const SolveTables& t, double2* rho, cudaStream_t stream) {
   const size_t smem = (size_t)kRho0Warps * 3 * t.nw2 * sizeof(double2);
-  cudaFuncSetAttribute(rho0_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared_memory(rho0_fp64_kernel, smem);
   rho0_fp64_kernel<<<(t.Nk + kRho0Warps - 1) / kRho0Warps, kRho0Warps * 32, smem, stream>>>(t, rho);
   return 1;
 }

@@ -32,6 +32,7 @@
 
 #include "dmma.cuh"
 #include "sbe_device.h"
+#include "smem_limit.h"
 #include "warp_reduce.cuh"
 
 namespace hhg {
@@ -929,7 +930,7 @@ bool plan_group_t(const SolveTables& t, int sm_count, LaunchShape* out, char* wh
   }
   auto kern = propagate_group_kernel<Real, EPT, NWc, NAXc, NJc, KM, WBc, KP, PG>;
   const size_t smem_max = bytes(best, box_sm, win_sm);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max);
+  allow_shared_memory(kern, smem_max);
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, best / KPG * G, smem_max);
   if (occ < 1) occ = 1;
@@ -973,7 +974,7 @@ int launch_group_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
     d.Gpre = Gpre;
     d.GWpre = GWpre;
     auto kern = propagate_group_kernel<Real, EPT, NWc, NAXc, NJc, KM, WBc, KP, true>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    allow_shared_memory(kern, s.smem);
     int launches = 0;
     for (int c0 = t.step0; c0 < t.step1; c0 += s.pre_chunk) {
       SolveTables tc = t;
@@ -988,7 +989,7 @@ int launch_group_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
     return launches;
   } else {
     auto kern = propagate_group_kernel<Real, EPT, NWc, NAXc, NJc, KM, WBc, KP, false>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    allow_shared_memory(kern, s.smem);
     kern<<<s.ctas, s.threads, s.smem, stream>>>(t, d, s.k_per_cta, s.group, s.box_sm, s.win_sm, s.vctas, rho, Jpart);
     return 1;
   }
@@ -998,7 +999,7 @@ template <typename Real, int EPT, int NWc, int NAXc, int NJc, bool KM = false, i
 int launch_group_batch_t(const BatchDesc* descs, const int2* items, int nitems, int* counter, int threads, size_t smem,
                          int sm_count, cudaStream_t stream) {
   auto kern = propagate_group_batch_kernel<Real, EPT, NWc, NAXc, NJc, KM, WBc, KP>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared_memory(kern, smem);
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem);
   if (occ < 1) occ = 1;
@@ -1012,8 +1013,7 @@ template <int NW, int NAX, int NJ, int KPC>
 bool plan_frag_t(const SolveTables& t, int sm_count, LaunchShape* out, char* why, int why_len) {
   using FG = frag::Geom<NW, NAX, NJ, KPC>;
   auto kern = frag::propagate_frag_kernel<NW, NAX, NJ, KPC>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG::BYTES) != cudaSuccess) {
-    cudaGetLastError();
+  if (!allow_shared_memory(kern, FG::BYTES)) {
     snprintf(why, why_len, "fragment kernel: %zu bytes of shared memory not available", FG::BYTES);
     return false;
   }
@@ -1053,7 +1053,7 @@ int launch_frag_t(const SolveTables& t, const GroupTables& gt, const LaunchShape
   d.Gpre = Gpre;
   d.GWpre = GWpre;
   auto kern = frag::propagate_frag_kernel<NW, NAX, NJ, KPC>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  allow_shared_memory(kern, s.smem);
   int launches = 0;
   for (int c0 = t.step0; c0 < t.step1; c0 += s.pre_chunk) {
     SolveTables tc = t;
@@ -1071,8 +1071,7 @@ template <int NW, int NAX, int NJ, int KPC, bool KM>
 bool plan_mtile_t(const SolveTables& t, int sm_count, LaunchShape* out, char* why, int why_len) {
   using FG = mtile::Geom<NW, NAX, NJ, KPC, KM>;
   auto kern = mtile::propagate_mtile_kernel<NW, NAX, NJ, KPC, KM>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG::BYTES) != cudaSuccess) {
-    cudaGetLastError();
+  if (!allow_shared_memory(kern, FG::BYTES)) {
     snprintf(why, why_len, "tile kernel: %zu bytes of shared memory not available", FG::BYTES);
     return false;
   }
@@ -1114,7 +1113,7 @@ int launch_mtile_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
   d.Gpre = Gpre;
   d.GWpre = GWpre;
   auto kern = mtile::propagate_mtile_kernel<NW, NAX, NJ, KPC, KM>;
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  allow_shared_memory(kern, s.smem);
   int launches = 0;
   for (int c0 = t.step0; c0 < t.step1; c0 += s.pre_chunk) {
     SolveTables tc = t;

@@ -38,6 +38,7 @@
 #include <stdexcept>
 
 #include "sbe_device.h"
+#include "smem_limit.h"
 
 namespace hhg {
 namespace {
@@ -595,7 +596,7 @@ bool plan_kcol(const SolveTables& t, int sm_count, LaunchShape* out, size_t smem
   // hide: 120 x 120 (240 tiles) 0.45 against 0.40, 200 x 200 (800 tiles, 4096 steps) 2.90 against 2.60.
   const int warps = 2 * ntiles <= 3 * sm_count ? 2 : 1;
   const KcolKernel kern = f.kern[warps - 1];
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+  allow_shared_memory(kern, f.smem);
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * warps, f.smem);
   if (occ < 1) return plan_kcol_any(t, sm_count, out, smem_max, parts_hint);
@@ -627,7 +628,7 @@ int launch_kcol(const SolveTables& t, const GroupTables& gt, const LaunchShape& 
     throw std::runtime_error("column-tile launch: needs its table scratch (GroupTables::pre)");
   const Form f = form_of(t);
   const KcolKernel kern = f.kern[s.threads / 32 - 1];
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  allow_shared_memory(kern, s.smem);
   double* tables[2] = {static_cast<double*>(gt.pre), static_cast<double*>(gt.pre) + (size_t)t.N2 * (s.pre_chunk * f.rec + f.col)};
   KcolArgs a{};
   a.t = t;

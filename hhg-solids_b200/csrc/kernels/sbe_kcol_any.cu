@@ -20,6 +20,7 @@
 
 #include "sbe_device.h"
 #include "sbe_herm2.cuh"
+#include "smem_limit.h"
 
 namespace hhg {
 namespace {
@@ -480,7 +481,7 @@ bool plan_kcol_any(const SolveTables& t, int sm_count, LaunchShape* out, size_t 
   const size_t smem = L.bytes(threads);
   if (smem > smem_max || threads > kKcolMaxThreads) return false;
   KcolKernel kern = kcol_kernel_for(t, half);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_shared_memory(kern, smem);
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem);
   if (occ < 1) return false;
@@ -503,7 +504,7 @@ bool plan_kcol_any(const SolveTables& t, int sm_count, LaunchShape* out, size_t 
 void launch_kcol_any(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
                  cudaStream_t stream) {
   KcolKernel kern = kcol_kernel_for(t, s.variant == 1);
-  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+  allow_shared_memory(kern, s.smem);
   kern<<<s.ctas, s.threads, s.smem, stream>>>(t, gt, s.k_per_cta, s.vctas, rho, Jpart);
 }
 
