@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "sbe_device.h"
+#include "smem_limit.h"
 
 namespace hhg {
 namespace {
@@ -217,12 +218,11 @@ int spectrum_device(const double2* J, int n, int count, double h, double2* S, do
   const int passes = (int)rad.size();
   double2* w = scratch + (size_t)count * n;
   roots_kernel<<<(n + 255) / 256, 256, 0, stream>>>(w, n);
-  if (n <= kBlockSamples) {
+  const size_t smem = 2 * (size_t)n * sizeof(double2);
+  if (n <= kBlockSamples && allow_shared_memory(stockham_block_kernel, smem)) {
     Radices r{};
     r.count = passes;
     for (int p = 0; p < passes; ++p) r.r[p] = rad[p];
-    const size_t smem = 2 * (size_t)n * sizeof(double2);
-    cudaFuncSetAttribute(stockham_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     stockham_block_kernel<<<count, kBlockThreads, smem, stream>>>(J, S, w, n, r, h);
     return cudaGetLastError() == cudaSuccess ? passes : -1;
   }
