@@ -165,9 +165,11 @@ __global__ void stockham_pass_kernel(const double2* in, double2* out, const doub
 // samples took 1 ms for any number of signals.)
 __global__ void harmonics_kernel(const double2* S, int n, int i0, int ni, int count, double tmax, double w0, int nh,
                                  double* I) {
-  const int gid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (gid >= count * nh) return;
-  const int b = gid / nh, hh = gid % nh;
+  // (in 64 bits: 2^27 values are 2^32 threads)
+  const long long gid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (gid >= (long long)count * nh) return;
+  const int b = (int)(gid / nh), hh = (int)(gid % nh);
   const double h = 2.0 * hh + 1.0;
   const double wmax = n * (2.0 * M_PI / tmax) / 2.0;
   const double step = n > 1 ? 2.0 * wmax / (double)(n - 1) : 0.0;

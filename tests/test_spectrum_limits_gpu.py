@@ -1,4 +1,5 @@
-"""Spectra at the limits of their launches: calls of different lengths from several threads."""
+"""Spectra at the limits of their launches: calls of different lengths from several threads, and more harmonic values
+than a 32-bit thread index counts."""
 import threading
 import time
 
@@ -38,3 +39,25 @@ def test_transforms_of_several_lengths_side_by_side():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_more_harmonic_values_than_2_to_the_27():
+    """A warp per value: 2^27 of them are 2^32 threads.  Eleven samples whose orders reach the last harmonic; the
+    expected sums take each sample's order (exact to 1e-7) to its window, and hold one sample each."""
+    from pySWE import pyswe
+
+    nh, n, tmax = (1 << 27) + 1000, 11, 1.0
+    top = 2 * nh - 1
+    lam = 600.0 * tmax * top / n  # the last sample has the last harmonic's order
+    rng = np.random.default_rng(5)
+    S = rng.standard_normal((1, n)) + 1j * rng.standard_normal((1, n))
+    order = np.linspace(-top, top, n)
+    near = np.rint(order).astype(np.int64)
+    held = [(int(near[i] // 2), abs(S[0, i]) ** 2) for i in range(n)
+            if near[i] > 0 and near[i] % 2 == 1 and abs(order[i] - near[i]) < 0.49]
+    assert np.all(np.abs(np.abs(order - near) - 0.5) > 1e-3) and len(held) >= 2 and held[-1][0] == nh - 1
+    I = pyswe.harmonic_intensities(S, tmax, lam, nh)[0]
+    where = np.flatnonzero(I)
+    assert where.tolist() == [k for k, _ in held]
+    for k, v in held:
+        assert abs(I[k] - v) <= 1e-14 * v
