@@ -682,28 +682,64 @@ size_t SWESim::footprint_estimate() const {
   const size_t nt_ = (size_t)std::max(2, (int)(s.tmax / s.dt));
   const size_t N1_ = (size_t)std::max(1, s.nr1), N2_ = (size_t)std::max(1, s.nr2);
   const size_t w2 = (size_t)m.nw * m.nw, ns = (size_t)std::max(1, m.nsites);
-  int np_ = 2;
-  for (int c = 0; c < m.nsites; ++c) np_ = std::max(np_, std::max(std::abs(m.R[3 * c]), std::abs(m.R[3 * c + 1])));
+  int m1 = 0, m2 = 0;  // extents of the model's cells
+  for (int c = 0; c < m.nsites; ++c) {
+    m1 = std::max(m1, std::abs(m.R[3 * c]));
+    m2 = std::max(m2, std::abs(m.R[3 * c + 1]));
+  }
+  const int np_ = std::max(2, std::max(m1, m2));
   const size_t box = (size_t)(2 * np_ + 1) * (2 * np_ + 1);
   int dev = device, sms = 148;
   if (dev < 0) cudaGetDevice(&dev);
   if (dev >= 0) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const size_t c16 = sizeof(double2);
-  size_t b = 2 * N1_ * N2_ * w2 * c16;                            // rho, rho0
-  b += 4 * (size_t)sms * nt_ * 3 * c16;                           // current partials (up to 4 CTAs per SM)
-  b += nt_ * (3 * c16 + 9 * sizeof(double));                      // J, field table
-  b += nt_ * (ns + hhg::kWindow) * c16;                           // Peierls phases of the listed cells
-  b += nt_ * 2 * (2 * np_ + 1) * c16 * 3 / 2;                     // P, FP64 and FP32
-  b += (4 * box + 4 * ns + 6 * hhg::kWindow) * w2 * c16 * 3 / 2;  // cell tables, both precisions
-  b += (N1_ + N2_) * c16 * 3 / 2 + (size_t(1) << 20);
   // Precomputed inner sums: 64 steps (2 x 64 + 1 points for the k-space solver) x N2 columns x (box
   // rows of H0 and r_a, window rows) x nw2.
   const size_t pre_pts = solver == 1 ? 2 * std::min<size_t>(64, nt_) + 1 : std::min<size_t>(64, nt_);
   // (The fragment kernel's: 8-column tiles of the elements i <= j, two k-steps per matrix, window coefficients.)
   const size_t tiles = (w2 + (size_t)m.nw + 7) / 8;
-  b += pre_pts * N2_ * std::max(((size_t)4 * (np_ + 1) + 12) * w2 * c16, (size_t)(4 + 3) * tiles * 512);
-  // Two orbitals: the column tables of 512 steps, two of up to 22 doubles and two axes' coefficients a step.
-  if (m.nw == 2) b += (std::min<size_t>(512, nt_) + 1) * N2_ * (2 * 22 + 2 * 32) * sizeof(double);
+  size_t pre = pre_pts * N2_ * std::max(((size_t)4 * (np_ + 1) + 12) * w2 * c16, (size_t)(4 + 3) * tiles * 512);
+  // Rows of current partials, one per CTA: up to 4 CTAs per SM.  The kernels of one and two orbitals have more (8 per SM
+  // for two orbitals on 300 x 300, 12 for one on 32 x 3000) and tables of their own: as the planner splits the model's
+  // whole box.
+  size_t rows = 4 * (size_t)sms;
+  if (m.nw <= 2 && N1_ >= 4 && N2_ >= 4 && N1_ % 2 == 0 && N2_ % 2 == 0 && N1_ * N2_ <= (size_t(1) << 30)) {
+    hhg::SolveTables q{};
+    q.nw = m.nw;
+    q.nw2 = (int)w2;
+    q.N1 = (int)N1_;
+    q.N2 = (int)N2_;
+    q.Nk = q.N1 * q.N2;
+    q.nt = q.step1 = (int)nt_;
+    q.row0 = std::max(0, req_row0);
+    q.row1 = req_row1 < 0 ? q.N1 : std::min(req_row1, q.N1);
+    q.kmode = solver;
+    q.hermitian = 1;
+    q.nax = (s.sx != 0.0) + (s.sy != 0.0) + (s.sz != 0.0);
+    q.ncell = m.nsites;
+    q.nwin = hhg::kWindow;
+    const int h1 = solver == 1 ? m2 : m1, h2 = solver == 1 ? m1 : m2;
+    q.b1lo = -std::min(h1, q.N1 / 2);
+    q.b2lo = -std::min(h2, q.N2 / 2);
+    q.b1n = 1 - 2 * q.b1lo;
+    q.b2n = 1 - 2 * q.b2lo;
+    q.np = np_;
+    for (q.nj = 1; q.nj <= 3 && q.row0 < q.row1; ++q.nj) {  // (current axes: known after the velocity tables)
+      hhg::LaunchShape sh{};
+      char why[256];
+      if (!hhg::plan_propagate(q, precision, sms, &sh, why, sizeof why)) continue;
+      rows = std::max(rows, (size_t)sh.vctas);
+      pre = std::max(pre, sh.pre_bytes);
+    }
+  }
+  const size_t pts = solver == 1 ? 2 * nt_ + 1 : nt_;             // evaluation points of the factor tables
+  size_t b = 2 * N1_ * N2_ * w2 * c16;                            // rho, rho0
+  b += rows * nt_ * 3 * c16 + pre;                                // current partials, precomputed sums
+  b += nt_ * (3 * c16 + 12 * sizeof(double));                     // J, field tables
+  b += pts * ((ns + hhg::kWindow) * c16 + 2 * sizeof(double));    // factors of the listed cells, stencil offsets
+  b += pts * 2 * (2 * np_ + 1) * c16 * 3 / 2;                     // P, FP64 and FP32
+  b += (4 * box + 4 * ns + 6 * hhg::kWindow) * w2 * c16 * 3 / 2;  // cell tables, both precisions
+  b += (N1_ + N2_) * c16 * 3 / 2 + (size_t(1) << 20);
   return b;
 }
 
