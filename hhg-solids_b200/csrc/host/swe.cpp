@@ -808,7 +808,6 @@ void SWESim::run() {
     drop_run_graph();
     last_launches = enqueue();
   } else {
-    if (run_graph && (run_graph_gen != generation || run_graph_hJ != hJ)) drop_run_graph();
     if (!run_graph) {
       cudaGraph_t g = nullptr;
       check_cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
@@ -824,8 +823,6 @@ void SWESim::run() {
       const cudaError_t e = cudaGraphInstantiate(&run_graph, g, 0);
       cudaGraphDestroy(g);
       check_cuda(e, "graph instantiate");
-      run_graph_gen = generation;
-      run_graph_hJ = hJ;
       graph_launches = n;
     }
     check_cuda(cudaGraphLaunch(run_graph, stream), "graph launch");

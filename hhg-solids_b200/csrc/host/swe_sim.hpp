@@ -139,11 +139,10 @@ struct SWESim {
   std::vector<hhg::cd> Jhist[3];
   float last_ms = 0.f, last_prop_ms = 0.f;
   // run()'s launch sequence (clear, propagate, reduce, copy the current out), launched directly by a setup's first
-  // run, captured by its second and replayed; rebuilt when a new setup or a new pinned buffer changes what it points at.
+  // run, captured by its second and replayed.  Everything it points at lasts as long as the setup: init() and release()
+  // drop it.
   cudaGraphExec_t run_graph = nullptr;
-  unsigned run_graph_gen = 0;
   unsigned first_run_gen = 0;  // the setup whose first run has been made
-  const double2* run_graph_hJ = nullptr;
   int graph_launches = 0;  // kernel launches inside run_graph
   void drop_run_graph() {
     if (run_graph) cudaGraphExecDestroy(run_graph);
