@@ -15,6 +15,7 @@
 // factors come from one table of the n-th roots: a radix-4093 pass was one thread with a sincospi per term.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <vector>
 
@@ -24,12 +25,27 @@
 namespace hhg {
 namespace {
 
+// The order axis of n samples: linspace(-wmax, wmax, n) / w0, its divisions made once on the host.
+struct OrderAxis {
+  int n;
+  double w0, wmax, step, per_step;
+};
+OrderAxis order_axis(int n, double tmax, double lambda_nm) {
+  OrderAxis x;
+  x.n = n;
+  x.w0 = 2.0 * M_PI * 300.0 / lambda_nm;
+  x.wmax = n * (2.0 * M_PI / tmax) / 2.0;
+  x.step = n > 1 ? 2.0 * x.wmax / (double)(n - 1) : 1.0;
+  x.per_step = 1.0 / x.step;
+  return x;
+}
+
 // Samples [lo, hi) that can hold orders between a and b: two more on either side than the axis says.
-__host__ __device__ inline void harmonic_window(int n, double tmax, double w0, double a, double b, int* lo, int* hi) {
-  const double wmax = n * (2.0 * M_PI / tmax) / 2.0, step = n > 1 ? 2.0 * wmax / (double)(n - 1) : 1.0;
-  const double x = floor((a * w0 + wmax) / step) - 2.0, y = ceil((b * w0 + wmax) / step) + 3.0;
-  *lo = x < 0.0 ? 0 : (x > (double)n ? n : (int)x);
-  *hi = y < 0.0 ? 0 : (y > (double)n ? n : (int)y);
+__host__ __device__ inline void harmonic_window(const OrderAxis& ax, double a, double b, int* lo, int* hi) {
+  const double n = (double)ax.n;
+  const double x = floor((a * ax.w0 + ax.wmax) * ax.per_step) - 2.0, y = ceil((b * ax.w0 + ax.wmax) * ax.per_step) + 3.0;
+  *lo = x < 0.0 ? 0 : (x > n ? ax.n : (int)x);
+  *hi = y < 0.0 ? 0 : (y > n ? ax.n : (int)y);
 }
 
 __device__ __forceinline__ double2 sp_mul(double2 a, double2 b) {
@@ -110,7 +126,7 @@ struct Radices {
   int count, r[30];
 };
 constexpr int kBlockSamples = 7040;  // two buffers of a signal in 220 KB of shared memory
-constexpr int kBlockThreads = 512;
+constexpr int kBlockThreads = 512;  // at most: a thread per sample of shorter signals
 
 // A block per signal, all passes in shared memory.
 __global__ void __launch_bounds__(kBlockThreads) stockham_block_kernel(const double2* J, double2* S, const double2* w,
@@ -126,10 +142,10 @@ __global__ void __launch_bounds__(kBlockThreads) stockham_block_kernel(const dou
     double2* dst = sp_buf + (size_t)(~p & 1) * n;
     // (a large first radix reads each input for every output: the gradient is formed once)
     if (first && R > 8) {
-      for (int i = threadIdx.x; i < n; i += kBlockThreads) sp_buf[i] = sp_grad_shifted(Jb, n, i, h);
+      for (int i = threadIdx.x; i < n; i += blockDim.x) sp_buf[i] = sp_grad_shifted(Jb, n, i, h);
       __syncthreads();
     }
-    for (int it = threadIdx.x; it < items; it += kBlockThreads)
+    for (int it = threadIdx.x; it < items; it += blockDim.x)
       stockham_item(
           it, n, R, Ns, w, [&](int i) { return first && R <= 8 ? sp_grad_shifted(Jb, n, i, h) : src[i]; },
           [&](int o, double2 v) {
@@ -159,35 +175,34 @@ __global__ void stockham_pass_kernel(const double2* in, double2* out, const doub
       [&](int o, double2 v) { dst[last ? (o + n / 2) % n : o] = v; });
 }
 
-// I[b][h'] for odd harmonics h = 2 h' + 1: sum of |S|^2 over order in (h - 1/2, h + 1/2).  A warp per value; the
-// samples of the window are found from the order axis (with a margin for its rounding) and each is tested as
-// written above.  S holds the samples i0 .. i0 + ni - 1 of each signal.  (A thread per value that tested all n
-// samples took 1 ms for any number of signals.)
-__global__ void harmonics_kernel(const double2* S, int n, int i0, int ni, int count, double tmax, double w0, int nh,
+// I[b][h'] for odd harmonics h = 2 h' + 1: sum of |S|^2 over order in (h - 1/2, h + 1/2).  `lanes` lanes per value, as
+// many as its window has samples, up to a warp; the samples of the window are found from the order axis (with a margin
+// for its rounding) and each is tested as written above.  S holds the samples i0 .. i0 + ni - 1 of each signal.
+// (A thread per value that tested all n samples took 1 ms for any number of signals; a warp per value whatever its
+// window 20.6 ms a call, copies included, for 300 000 signals of 3 samples and 25 values, against 18.2.)
+__global__ void harmonics_kernel(const double2* S, OrderAxis ax, int i0, int ni, long long values, int nh, int lanes,
                                  double* I) {
-  // (in 64 bits: 2^27 values are 2^32 threads)
-  const long long gid = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (gid >= (long long)count * nh) return;
-  const int b = (int)(gid / nh), hh = (int)(gid % nh);
-  const double h = 2.0 * hh + 1.0;
-  const double wmax = n * (2.0 * M_PI / tmax) / 2.0;
-  const double step = n > 1 ? 2.0 * wmax / (double)(n - 1) : 0.0;
-  int lo, hi;
-  harmonic_window(n, tmax, w0, h - 0.5, h + 0.5, &lo, &hi);
-  lo = max(lo, i0);
-  hi = min(hi, i0 + ni);
+  // (in 64 bits: 2^27 values of a warp each are 2^32 threads)
+  const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+  const int lane = threadIdx.x & (lanes - 1);
   double acc = 0.0;
-  for (int i = lo + lane; i < hi; i += 32) {
-    const double order = (-wmax + step * i) / w0;
-    if (order > h - 0.5 && order < h + 0.5) {
-      const double2 s = S[(size_t)b * ni + (i - i0)];
-      acc += s.x * s.x + s.y * s.y;
+  if (gid < values) {
+    const long long b = gid / nh;
+    const double h = 2.0 * (double)(gid - b * nh) + 1.0;
+    int lo, hi;
+    harmonic_window(ax, h - 0.5, h + 0.5, &lo, &hi);
+    lo = max(lo, i0);
+    hi = min(hi, i0 + ni);
+    for (int i = lo + lane; i < hi; i += lanes) {
+      const double order = (-ax.wmax + ax.step * i) / ax.w0;
+      if (order > h - 0.5 && order < h + 0.5) {
+        const double2 s = S[(size_t)b * ni + (i - i0)];
+        acc += s.x * s.x + s.y * s.y;
+      }
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) I[gid] = acc;
+  for (int o = lanes / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  if (gid < values && lane == 0) I[gid] = acc;
 }
 
 std::vector<int> factor_radices(int n) {
@@ -225,7 +240,7 @@ int spectrum_device(const double2* J, int n, int count, double h, double2* S, do
     Radices r{};
     r.count = passes;
     for (int p = 0; p < passes; ++p) r.r[p] = rad[p];
-    stockham_block_kernel<<<count, kBlockThreads, smem, stream>>>(J, S, w, n, r, h);
+    stockham_block_kernel<<<count, std::min(kBlockThreads, (n + 31) / 32 * 32), smem, stream>>>(J, S, w, n, r, h);
     return cudaGetLastError() == cudaSuccess ? passes : -1;
   }
   // Ping-pong between S and scratch so that the last pass lands in S.
@@ -248,7 +263,7 @@ int spectrum_device(const double2* J, int n, int count, double h, double2* S, do
 
 void harmonics_range(int n, double tmax, double lambda_nm, int nh, int* i0, int* ni) {
   int lo, hi;
-  harmonic_window(n, tmax, 2.0 * M_PI * 300.0 / lambda_nm, 0.5, 2.0 * nh - 0.5, &lo, &hi);
+  harmonic_window(order_axis(n, tmax, lambda_nm), 0.5, 2.0 * nh - 0.5, &lo, &hi);
   *i0 = lo;
   *ni = hi > lo ? hi - lo : 0;
 }
@@ -256,9 +271,12 @@ void harmonics_range(int n, double tmax, double lambda_nm, int nh, int* i0, int*
 int harmonics_device(const double2* S, int n, int i0, int ni, int count, double tmax, double lambda_nm, int nh, double* I,
                      cudaStream_t stream) {
   if (n < 2 || count < 1 || nh < 1 || tmax <= 0.0 || lambda_nm <= 0.0) return -1;
-  const double w0 = 2.0 * M_PI * 300.0 / lambda_nm;
-  const long long warps = (long long)count * nh;
-  harmonics_kernel<<<(unsigned)((warps + 3) / 4), 128, 0, stream>>>(S, n, i0, ni, count, tmax, w0, nh, I);
+  const OrderAxis ax = order_axis(n, tmax, lambda_nm);
+  const double window = ax.w0 * ax.per_step + 6.0;  // samples tested per value, at most
+  int lanes = 1;
+  while (lanes < 32 && lanes < window) lanes *= 2;
+  const long long values = (long long)count * nh;
+  harmonics_kernel<<<(unsigned)((values * lanes + 127) / 128), 128, 0, stream>>>(S, ax, i0, ni, values, nh, lanes, I);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

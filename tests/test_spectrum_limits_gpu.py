@@ -1,5 +1,5 @@
-"""Spectra at the limits of their launches: calls of different lengths from several threads, and more harmonic values
-than a 32-bit thread index counts."""
+"""Spectra at the limits of their launches: calls of different lengths from several threads, many signals of a few
+samples, and more harmonic values than a 32-bit thread index counts."""
 import threading
 import time
 
@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from conftest import rel_l2
-from test_spectrum_gpu import numpy_spectrum
+from test_spectrum_gpu import numpy_harmonics, numpy_spectrum
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +61,19 @@ def test_more_harmonic_values_than_2_to_the_27():
     assert where.tolist() == [k for k, _ in held]
     for k, v in held:
         assert abs(I[k] - v) <= 1e-14 * v
+
+
+@pytest.mark.parametrize("n,count,tmax,nh", [(2, 4001, 0.04, 25), (3, 1000, 0.06, 7), (8, 2000, 0.16, 25), (16, 500, 0.32, 25),
+                                             (31, 300, 2.0, 3), (33, 300, 40.0, 2), (130, 99, 9.0, 40)])
+def test_many_short_signals(n, count, tmax, nh):
+    """Blocks of a warp up to 16 of them, windows of none to some samples, uploaded whole or in part.  Transforms
+    1e-13 relative L2 (below 1e-15 x log2 n of rounding), sums of non-negative terms 1e-12."""
+    from pySWE import pyswe
+
+    rng = np.random.default_rng(n)
+    J = rng.standard_normal((count, n)) + 1j * rng.standard_normal((count, n))
+    S, ref = pyswe.spectrum(J, tmax / n), numpy_spectrum(J, tmax / n)
+    assert max(rel_l2(S[a], ref[a]) for a in range(count)) < 1e-13
+    I, I_ref = pyswe.harmonic_intensities(S, tmax, 3000.0, nh), numpy_harmonics(S, tmax, 3000.0, nh)
+    assert np.array_equal(I == 0, I_ref == 0)
+    assert np.all(np.abs(I - I_ref) <= 1e-12 * I_ref)
