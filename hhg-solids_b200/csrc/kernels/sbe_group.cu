@@ -1067,10 +1067,10 @@ int launch_frag_t(const SolveTables& t, const GroupTables& gt, const LaunchShape
 }
 
 // Mixed-form tile kernel: precomputed inner sums, compiled 7x7 box, KPC k-points per CTA (half a warp each).
-template <int NW, int NAX, int NJ, int KPC, bool KM>
+template <int NW, int NAX, int NJ, int KPC, bool KM, bool PACK>
 bool plan_mtile_t(const SolveTables& t, int sm_count, LaunchShape* out, char* why, int why_len) {
   using FG = mtile::Geom<NW, NAX, NJ, KPC, KM>;
-  auto kern = mtile::propagate_mtile_kernel<NW, NAX, NJ, KPC, KM>;
+  auto kern = mtile::propagate_mtile_kernel<NW, NAX, NJ, KPC, KM, PACK>;
   if (!allow_shared_memory(kern, FG::BYTES)) {
     snprintf(why, why_len, "tile kernel: %zu bytes of shared memory not available", FG::BYTES);
     return false;
@@ -1099,7 +1099,7 @@ bool plan_mtile_t(const SolveTables& t, int sm_count, LaunchShape* out, char* wh
   return true;
 }
 
-template <int NW, int NAX, int NJ, int KPC, bool KM>
+template <int NW, int NAX, int NJ, int KPC, bool KM, bool PACK>
 int launch_mtile_t(const SolveTables& t, const GroupTables& gt, const LaunchShape& s, double2* rho, double2* Jpart,
                    cudaStream_t stream) {
   using FG = mtile::Geom<NW, NAX, NJ, KPC, KM>;
@@ -1112,7 +1112,7 @@ int launch_mtile_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
   double2* GWpre = reinterpret_cast<double2*>(Gpre + npts_max * t.N2 * gbuf);
   d.Gpre = Gpre;
   d.GWpre = GWpre;
-  auto kern = mtile::propagate_mtile_kernel<NW, NAX, NJ, KPC, KM>;
+  auto kern = mtile::propagate_mtile_kernel<NW, NAX, NJ, KPC, KM, PACK>;
   allow_shared_memory(kern, s.smem);
   int launches = 0;
   for (int c0 = t.step0; c0 < t.step1; c0 += s.pre_chunk) {
@@ -1129,34 +1129,44 @@ int launch_mtile_t(const SolveTables& t, const GroupTables& gt, const LaunchShap
 
 struct MtileVariant {
   int nw, nax, nj, kpc;
-  bool km;
+  bool km, pack;
   bool (*plan)(const SolveTables&, int, LaunchShape*, char*, int);
   int (*launch)(const SolveTables&, const GroupTables&, const LaunchShape&, double2*, double2*, cudaStream_t);
 };
-#define HHG_MTILE_VARIANT(NW, NAX, NJ, KPC, KM) \
-  {NW, NAX, NJ, KPC, KM, plan_mtile_t<NW, NAX, NJ, KPC, KM>, launch_mtile_t<NW, NAX, NJ, KPC, KM>}
+#define HHG_MTILE_VARIANT(NW, NAX, NJ, KPC, KM, PACK) \
+  {NW, NAX, NJ, KPC, KM, PACK, plan_mtile_t<NW, NAX, NJ, KPC, KM, PACK>, launch_mtile_t<NW, NAX, NJ, KPC, KM, PACK>}
 // (12 x 12 frame: 8 k-points per CTA; 6 x 6 frame: 32.  The k-space solver's ring of four inner-sum
 // slots leaves three CTAs per SM for 11 orbitals with one field axis, two for its other 12 x 12 shapes,
 // which still run 1.2-2x faster than the element-group kernel.)
 const MtileVariant kMtileVariants[] = {
-    HHG_MTILE_VARIANT(11, 1, 2, 8, false), HHG_MTILE_VARIANT(11, 2, 2, 8, false),
-    HHG_MTILE_VARIANT(12, 1, 2, 8, false), HHG_MTILE_VARIANT(12, 2, 2, 8, false),
-    HHG_MTILE_VARIANT(11, 1, 2, 8, true),  HHG_MTILE_VARIANT(11, 2, 2, 8, true),
-    HHG_MTILE_VARIANT(12, 1, 2, 8, true),  HHG_MTILE_VARIANT(12, 2, 2, 8, true),
-    HHG_MTILE_VARIANT(6, 1, 2, 32, false),  HHG_MTILE_VARIANT(6, 2, 2, 32, false),
-    HHG_MTILE_VARIANT(6, 1, 2, 32, true),   HHG_MTILE_VARIANT(6, 2, 2, 32, true),
+    HHG_MTILE_VARIANT(11, 1, 2, 8, false, true), HHG_MTILE_VARIANT(11, 2, 2, 8, false, true),
+    HHG_MTILE_VARIANT(12, 1, 2, 8, false, true), HHG_MTILE_VARIANT(12, 2, 2, 8, false, true),
+    HHG_MTILE_VARIANT(11, 1, 2, 8, true, true),  HHG_MTILE_VARIANT(11, 2, 2, 8, true, true),
+    HHG_MTILE_VARIANT(12, 1, 2, 8, true, true),  HHG_MTILE_VARIANT(12, 2, 2, 8, true, true),
+    HHG_MTILE_VARIANT(6, 1, 2, 32, false, true), HHG_MTILE_VARIANT(6, 2, 2, 32, false, true),
+    HHG_MTILE_VARIANT(6, 1, 2, 32, true, true),  HHG_MTILE_VARIANT(6, 2, 2, 32, true, true),
+    HHG_MTILE_VARIANT(11, 1, 2, 8, false, false), HHG_MTILE_VARIANT(11, 1, 2, 8, true, false),
+    HHG_MTILE_VARIANT(12, 1, 2, 8, false, false), HHG_MTILE_VARIANT(12, 1, 2, 8, true, false),
+    HHG_MTILE_VARIANT(6, 1, 2, 32, false, false), HHG_MTILE_VARIANT(6, 1, 2, 32, true, false),
 };
 #undef HHG_MTILE_VARIANT
 
 // The tile kernel for a mixed-form solve (Hermitian halved 7x7 box; either solver), or null.
 // HHG_MTILE=0 turns it off (measurements): the element-group kernel then runs the solve.
-const MtileVariant* find_mtile(const SolveTables& t) {
+// The commutator product is in packed FP32 pairs, except (same bits) with one field axis and no more tiles than SMs: a
+// CTA alone on its SM has issue slots to spare, which are what packing saves.  1024 steps, packed / scalar: 20 x 20
+// 6 orbitals 5.52 / 5.21 ms, 11 orbitals 6.35 / 6.26, 12 orbitals 6.28 / 6.09; with more tiles, 40 x 40, 11 orbitals
+// 7.82 / 8.15, 12 orbitals 8.04 / 8.53; with few tiles and two axes, 30 x 30, 11 orbitals 7.12 / 7.15.
+const MtileVariant* find_mtile(const SolveTables& t, int sm_count) {
   if (const char* off = std::getenv("HHG_MTILE"))
     if (off[0] == '0') return nullptr;
   const GroupGeom gg = group_geom(t);
   if (!t.hermitian || !gg.half || t.b1n != 7 || t.b2n != 7) return nullptr;
-  for (const MtileVariant& v : kMtileVariants)
-    if (v.nw == t.nw && v.nax == t.nax && v.nj == t.nj && v.km == (t.kmode != 0)) return &v;
+  for (const MtileVariant& v : kMtileVariants) {
+    if (v.nw != t.nw || v.nax != t.nax || v.nj != t.nj || v.km != (t.kmode != 0)) continue;
+    const long ntiles = (long)t.N2 * ((t.row1 - t.row0 + v.kpc - 1) / v.kpc);
+    if (v.pack != (t.nax == 1 && ntiles <= sm_count)) return &v;
+  }
   return nullptr;
 }
 
@@ -1287,7 +1297,7 @@ bool plan_group(const SolveTables& t, int precision, int sm_count, LaunchShape* 
       if (f->plan(t, sm_count, out, why, why_len)) return true;
     }
   if (precision == 1)
-    if (const MtileVariant* m = find_mtile(t)) {
+    if (const MtileVariant* m = find_mtile(t, sm_count)) {
       out->variant = (int)(m - kMtileVariants);
       if (m->plan(t, sm_count, out, why, why_len)) return true;
     }

@@ -125,7 +125,8 @@ struct Geom {
 // KM: the reference's k-space solver (src/solver_kspace.cpp:167-270): the stages see H at points
 // 2 ti (t), 2 ti + 1 (t + dt/2) and 2 ti + 2 (t + dt) of the interpolation tables; the outer sums of
 // 2 ti + 2 stay in registers for the next step's first stage, and the window has no phase.
-template <int NW, int NAX, int NJ, int KPC, bool KM = false>
+// PACK: the product in packed pairs; else in scalar operations (the planner's rule says where each is the faster).
+template <int NW, int NAX, int NJ, int KPC, bool KM, bool PACK>
 __global__ void __launch_bounds__(128, 3)
     propagate_mtile_kernel(SolveTables t, GroupData<float> d, int vctas, double2* rho, double2* Jpart) {
   using FG = Geom<NW, NAX, NJ, KPC, KM>;
@@ -432,10 +433,10 @@ __global__ void __launch_bounds__(128, 3)
           }
           __syncwarp();
           // P = H X on the tile: P(i, j) = sum_l H(i, l) X(l, j), H(i, l) from row l of the transposed H.
-          // Each complex multiply-add is two packed ones, h.x (x, y) then h.y (-y, x): the roundings and their
-          // order of four scalar ones.
           float2 P[9];
-          {
+          if constexpr (PACK) {
+            // Each complex multiply-add is two packed ones, h.x (x, y) then h.y (-y, x): the roundings and their
+            // order of four scalar ones.
             F2 acc[9];
 #pragma unroll
             for (int u = 0; u < 9; ++u) acc[u] = pack2(0.f, 0.f);
@@ -460,6 +461,19 @@ __global__ void __launch_bounds__(128, 3)
             }
 #pragma unroll
             for (int u = 0; u < 9; ++u) P[u] = unpack2(acc[u]);
+          } else {
+#pragma unroll
+            for (int u = 0; u < 9; ++u) P[u] = fzero;
+#pragma unroll
+            for (int l = 0; l < NW; ++l) {
+              const float2* hr = Hk + l * HMS + i0;
+              const float2* xr = Xk + l * MS + j0;
+              const float2 h[3] = {hr[0], hr[1], hr[2]}, x[3] = {xr[0], xr[1], xr[2]};
+#pragma unroll
+              for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) P[3 * a + c] = fmac(h[a], x[c], P[3 * a + c]);
+            }
           }
           __syncwarp();  // every lane of the k-point has read X and H
           if constexpr (!FG::SHFL) {
