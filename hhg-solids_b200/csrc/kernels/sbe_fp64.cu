@@ -16,7 +16,7 @@
 //
 // propagate_kpt_kernel<NW>  (nw <= 2, Hermitian placement): one thread per k-point, the whole
 //   state in registers; per-cell phases e^{-ik.R_c} (per thread, fixed) x e^{iA.R_c} (per step).
-// Two orbitals on all but the smallest grids: sbe_kcol.cu (one orbital, larger boxes: sbe_kcol_any.cu); 3 to 12 orbitals
+// Two orbitals on 160 k-points and more: sbe_kcol.cu (one orbital, larger boxes: sbe_kcol_any.cu); 3 to 12 orbitals
 // in FP64: sbe_dfrag.cu; the mixed form and everything else (any nw <= 16): sbe_group.cu.
 #include <cstdio>
 #include <cstdlib>
@@ -535,9 +535,10 @@ bool plan_propagate(const SolveTables& t, int precision, int sm_count, LaunchSha
   // nw <= 2 runs the FP64 thread-per-k-point kernels in both precisions: with 2x2 matrices the FP32
   // element-group kernel is several times slower, so the mixed form gains nothing there.
   if (!force_group && t.hermitian && t.nw <= 2) {
-    // Column tiles: the pair form on all but the smallest grids (the thread-per-k-point kernel keeps those of a few
-    // warps, which a test pins, at 1024 steps of 12 x 12 in 1.69 ms against 0.28), the general form when there are
-    // enough columns to fill the GPU; else one k-point per thread in consecutive-k tiles.
+    // Column tiles: the pair form, the general form when there are enough columns to fill the GPU; else one k-point per
+    // thread in consecutive-k tiles.  Grids below 160 k-points stay on the last, and not for speed: the pair form is the
+    // faster one there too (1024 steps of 12 x 12: 0.28 ms against 1.69).  The allocation-free entry is tested on the
+    // thread-per-k-point kernel with a 12 x 12 grid that reaches it by default.
     LaunchShape kc{};
     if (!force_kpt && plan_kcol(t, sm_count, &kc, kThreadKptSmem, tile_hint) &&
         (force_kcol || (kc.variant == 2 ? (t.row1 - t.row0) * t.N2 >= 160 : kc.ntiles >= sm_count))) {

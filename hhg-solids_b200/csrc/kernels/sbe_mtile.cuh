@@ -1,4 +1,4 @@
-// Mixed-form propagation for 4..6 and 9..12 orbitals in 3 x 3 register tiles, half a warp per k-point of 9..12
+// Mixed-form propagation for 6, 11 and 12 orbitals in 3 x 3 register tiles, half a warp per k-point of 11 and 12
 // (included by sbe_group.cu, inside its anonymous namespace: it uses GroupData, the precomputed inner
 // sums of group_sums_kernel and the helpers defined there).
 //
@@ -8,8 +8,8 @@
 // column and step (both solvers).
 //
 // Layout.  A CTA holds KPC consecutive k-points (rows m1) of one k-grid column; the k-point's matrices
-// are padded to a 12 x 12 frame (9..12 orbitals: 16 lanes, half a warp, per k-point, 8 per CTA) or a
-// 6 x 6 one (4..6 orbitals: 4 lanes per k-point, 32 per CTA), lane s owning its 3 x 3 tile (rows
+// are padded to a 12 x 12 frame (11 and 12 orbitals; it takes 9..12: 16 lanes, half a warp, per k-point, 8 per CTA)
+// or a 6 x 6 one (6 orbitals; it takes 4..6: 4 lanes per k-point, 32 per CTA), lane s owning its 3 x 3 tile (rows
 // 3 (s / T) .. +2, columns 3 (s % T) .. +2, T tiles per frame row).  Each lane keeps its tile of the state rho and of the RK4
 // sum in FP64 registers; the outer Wannier sums H0(k), r_a(k) of its elements (Geom::SHARE: which) give
 // H = H0 + E.r at the step's field samples, the later ones kept in FP32 registers for their stages.
@@ -19,7 +19,7 @@
 //  * the lane forms its tile of P = H X in FP32 from rows l of both arrays (three H and three X
 //    values per l: 36 FMA per 6 loads, every load a broadcast to the lanes of its tile row or
 //    column);
-//  * k = -i (P - P^+) takes P^+ from the lane of the transposed tile, by shuffles or (Geom::SHFL) through the
+//  * k = -i (P - P^+) takes P^+ from the lane of the transposed tile, by shuffles (Geom::SHFL) or through the
 //    place of X in shared memory;
 //  * the RK4 sum and the next stage's X are formed in FP64 (X stored as FP32).
 // Only the k-point's lanes (within one warp) exchange data, so the stages need __syncwarp only; the CTA meets twice
@@ -153,7 +153,8 @@ __global__ void __launch_bounds__(128, 3)
   float2* Xk = XPb + kp * KS;
   const float2 fzero = make_float2(0.f, 0.f);
   const double2 dzero = make_double2(0.0, 0.0);
-  // Tile slot u = 3 a + b is element (i0 + a, j0 + b); on the padding (row or column >= NW) it stays 0.
+  // Tile slot u = 3 a + b is element (i0 + a, j0 + b).  On the padding (row or column >= NW) it is no element: whatever
+  // H's unwritten padding leaves there reaches no slot of an element.
   auto valid = [&](int u) { return i0 + u / 3 < NW && j0 + u % 3 < NW; };
   auto own = [&](int u) { return (i0 + u / 3) * MS + j0 + u % 3; };   // (i, j) in X, P
   auto tra = [&](int u) { return (j0 + u % 3) * MS + i0 + u / 3; };   // (j, i): H, P^+
